@@ -225,6 +225,51 @@ at::Tensor spectral_weights(int M, int N, double wv_scale, at::Device device) {
   return out;
 }
 
+// table of a side for the fast transforms, on the host
+at::Tensor fft_twiddles(int n) {
+  TORCH_CHECK(dp_fft_supported(n, n), "fft_twiddles: unsupported side ", n);
+  auto out = at::empty({4 * (int64_t)n}, at::TensorOptions().dtype(at::kFloat));
+  DP_CALL(dp_fft_twiddles(n, ptr<float>(out)));
+  return out;
+}
+
+static void check_fft(const at::Tensor& x, const at::Tensor& tw_m, const at::Tensor& tw_n) {
+  CHECK_CUDA_T(x); CHECK_CONTIG(x); CHECK_F32(x);
+  TORCH_CHECK(x.dim() == 2, "the map must be two-dimensional");
+  for (auto* t : {&tw_m, &tw_n}) { CHECK_FLAT(*t); CHECK_F32(*t); }
+  TORCH_CHECK(tw_m.numel() == 4 * x.size(0) && tw_n.numel() == 4 * x.size(1), "twiddle tables of other sides");
+}
+
+void transform_fft(int kind, at::Tensor x, at::Tensor tw_m, at::Tensor tw_n, at::Tensor out) {
+  check_fft(x, tw_m, tw_n);
+  CHECK_CUDA_T(out); CHECK_CONTIG(out); CHECK_F32(out);
+  TORCH_CHECK(out.numel() == x.numel(), "transform_fft: output of another size");
+  c10::cuda::CUDAGuard guard(x.device());
+  auto work = at::empty_like(x);
+  DP_CALL(dp_transform_fft(kind, ptr<float>(x), (int)x.size(0), (int)x.size(1), ptr<float>(tw_m), ptr<float>(tw_n),
+                           ptr<float>(work), ptr<float>(out), cur_stream()));
+}
+
+// the solve into ex, ey (both or neither) and energy [1]; work: 3 M N floats
+void poisson_fft(at::Tensor rho, double rho_scale, double wv_scale, at::Tensor tw_m, at::Tensor tw_n,
+                 c10::optional<at::Tensor> work, c10::optional<at::Tensor> ex, c10::optional<at::Tensor> ey,
+                 at::Tensor energy, bool want_energy) {
+  check_fft(rho, tw_m, tw_n);
+  TORCH_CHECK(energy.is_cuda() && energy.scalar_type() == at::kDouble && energy.numel() >= 1, "energy must be float64");
+  c10::cuda::CUDAGuard guard(rho.device());
+  at::Tensor w = work.has_value() ? *work : at::empty({3 * rho.numel()}, rho.options());
+  CHECK_CUDA_T(w); CHECK_CONTIG(w); CHECK_F32(w);
+  TORCH_CHECK(w.numel() >= 3 * rho.numel(), "poisson_fft: work smaller than three maps");
+  for (auto* t : {&ex, &ey})
+    if (t->has_value())
+      TORCH_CHECK((*t)->is_cuda() && (*t)->is_contiguous() && (*t)->scalar_type() == at::kFloat &&
+                      (*t)->numel() == rho.numel(),
+                  "poisson_fft: a field map must be a contiguous float32 map of rho's size");
+  DP_CALL(dp_poisson_fft(ptr<float>(rho), (int)rho.size(0), (int)rho.size(1), (float)rho_scale, (float)wv_scale,
+                         ptr<float>(tw_m), ptr<float>(tw_n), ptr<float>(w), optr<float>(ex), optr<float>(ey), nullptr,
+                         ptr<double>(energy), want_energy ? 1 : 0, cur_stream()));
+}
+
 int tc_status() {
   int s = 0;
   DP_CALL(dp_tc_status(&s));
@@ -664,6 +709,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("electric_force", &electric_force);
   m.def("transform_gemm", &transform_gemm);
   m.def("prepare_operand", &prepare_operand);
+  m.def("fft_supported", [](int M, int N) { return dp_fft_supported(M, N) != 0; });
+  m.def("fft_twiddles", &fft_twiddles);
+  m.def("transform_fft", &transform_fft);
+  m.def("poisson_fft", &poisson_fft, py::arg("rho"), py::arg("rho_scale"), py::arg("wv_scale"), py::arg("tw_m"),
+        py::arg("tw_n"), py::arg("work"), py::arg("ex"), py::arg("ey"), py::arg("energy"), py::arg("want_energy"));
   m.def("tc_status", &tc_status);
   m.def("trial_metrics", [](at::Tensor hpwl, at::Tensor overflow2, at::Tensor state, at::Tensor obj, at::Tensor wl,
                             at::Tensor energy, at::Tensor out8) {

@@ -99,6 +99,12 @@ int opt_in_smem(Kernel kernel, int bytes, const char* who) {
   return DP_OK;
 }
 
+// the fast transforms' side of dp_tc_status / dp_tc_set_wait_budget /
+// dp_tc_set_skip_loads (fft.cu); each returns a cudaError_t
+int fft_take_status(int* out);  // leaves *out when no wait expired; clears the word
+int fft_set_wait_budget(long long cycles);
+int fft_set_skip_loads(int skip);
+
 // grid size for a grid-stride elementwise kernel: a multiple of the SM count
 inline int grid_for(long long n, int threads, int per_sm = 8) {
   long long blocks = (n + threads - 1) / threads;

@@ -57,7 +57,7 @@ __device__ __forceinline__ void spectral_weights(const EpiParams& p, int u, int 
   float wv = __fmul_rn(__fmul_rn((float)v, p.two_pi_over_n), p.wv_scale);
   float d = __fadd_rn(__fmul_rn(wu, wu), __fmul_rn(wv, wv));
   if (u == 0 && v == 0) d = 1.0f;
-  float inv = __fdiv_rn(1.0f, d);
+  float inv = __frcp_rn(d);  // correctly rounded, as 1 / d is
   if (u == 0 && v == 0) inv = 0.0f;
   winv = inv;
   wx = __fmul_rn(__fmul_rn(wu, inv), 0.5f);

@@ -406,13 +406,14 @@ int launch_tc_gemm(int precision, int M, int N, int K, const dp_gemm_problem* pr
 
 }  // namespace dpb
 
-// Reads and clears the device-side status word of the tensor-core kernels
-// (0 = no bounded wait expired).  Synchronises the device.
+// Reads and clears the device-side status words of the tensor-core kernels and
+// the fast transforms (0 = no bounded wait expired).  Synchronises the device.
 extern "C" int dp_tc_status(int* status_out) {
   DP_REQUIRE(status_out, "dp_tc_status: null output");
   int zero = 0;
   cudaError_t e = cudaMemcpyFromSymbol(status_out, dpb::g_tc_status, sizeof(int));
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(dpb::g_tc_status, &zero, sizeof(int));
+  if (e == cudaSuccess) e = (cudaError_t)dpb::fft_take_status(status_out);
   if (e != cudaSuccess) {
     dpb::set_error("dp_tc_status: %s", cudaGetErrorString(e));
     return DP_ERR_CUDA;
@@ -423,6 +424,7 @@ extern "C" int dp_tc_status(int* status_out) {
 extern "C" int dp_tc_set_wait_budget(long long cycles) {
   DP_REQUIRE(cycles > 0, "dp_tc_set_wait_budget: the budget must be positive");
   cudaError_t e = cudaMemcpyToSymbol(dpb::g_tc_wait_budget, &cycles, sizeof(long long));
+  if (e == cudaSuccess) e = (cudaError_t)dpb::fft_set_wait_budget(cycles);
   if (e != cudaSuccess) {
     dpb::set_error("dp_tc_set_wait_budget: %s", cudaGetErrorString(e));
     return DP_ERR_CUDA;
@@ -433,6 +435,7 @@ extern "C" int dp_tc_set_wait_budget(long long cycles) {
 extern "C" int dp_tc_set_skip_loads(int skip) {
   const int v = skip ? 1 : 0;
   cudaError_t e = cudaMemcpyToSymbol(dpb::g_tc_skip_loads, &v, sizeof(int));
+  if (e == cudaSuccess) e = (cudaError_t)dpb::fft_set_skip_loads(v);
   if (e != cudaSuccess) {
     dpb::set_error("dp_tc_set_skip_loads: %s", cudaGetErrorString(e));
     return DP_ERR_CUDA;

@@ -18,7 +18,10 @@ the spectral weights in the epilogue, the two right products batched in one
 launch, and the two left products batched with the Ex/Ey stores.  The energy
 is summed in the spectral domain by the second launch's epilogue,
   sum_xy rho IDCT2(a winv) = M N sum_uv w_u w_v winv_uv a_uv^2 (w_0 = 1/2),
-so the potential map is never formed.
+so the potential map is never formed.  In fp32 and split_bf16 on power-of-two
+grids the solve runs as fast transforms in three launches instead
+(csrc/fft.cu, dct2_fft2.fft_serves): rows; columns, weights, energy and the
+inverse column transforms; rows.
 Backward: the hand-written adjoint ``-electric_force`` (reference :219-275).
 
 The modules (``ElectricOverflow``, ``ElectricPotential``) keep a spatial
@@ -42,7 +45,7 @@ from torch.autograd import Function
 
 from ._native import C, precision_code, require_cuda
 from .dct2_fft2 import (DCT2, EPI_ENERGY, EPI_SPECTRAL, EPI_STORE, EPI_STORE_T, IDCT2, IDCT_IDXST, IDXST_IDCT,
-                        Operand, get_exact_expk, transform_matrices)
+                        Operand, fft_serves, fft_table, get_exact_expk, transform_matrices)
 
 logger = logging.getLogger(__name__)
 
@@ -72,15 +75,30 @@ class PoissonWorkspace(object):
     which then allocates nothing.  The returned field maps and energy are the
     workspace's own buffers, overwritten by the next solve."""
 
-    def __init__(self, M, N, prec, device):
+    def __init__(self, M, N, prec, device, fast=True):
+        """fast False: a workspace of the matrix products, also where the fast
+        transforms would serve the map."""
         self.key = (M, N, prec)
+        self.ex = torch.empty(M, N, dtype=torch.float32, device=device)
+        self.ey = torch.empty(M, N, dtype=torch.float32, device=device)
+        self.energy = torch.zeros(1, dtype=torch.float64, device=device)
+        self.fft_work = None
+        self.rho = self.t1 = self.spec = self.us = None
+        if fast and fft_serves(self.ex, prec):
+            self.fft_work = torch.empty(3 * M * N, dtype=torch.float32, device=device)
+        else:
+            self.products()
+
+    def products(self):
+        """Allocates the operands of the matrix products, once (a workspace of
+        the fast transforms needs them only for a map those do not take)."""
+        if self.t1 is not None:
+            return
+        (M, N, prec), device = self.key, self.ex.device
         self.rho = Operand((M, N), prec, device) if prec != 0 else None
         self.t1 = Operand((N, M), prec, device)
         self.spec = [Operand((M, N), prec, device) for _ in range(2)]
         self.us = [Operand((N, M), prec, device) for _ in range(2)]
-        self.ex = torch.empty(M, N, dtype=torch.float32, device=device)
-        self.ey = torch.empty(M, N, dtype=torch.float32, device=device)
-        self.energy = torch.zeros(1, dtype=torch.float64, device=device)
 
     def check(self, M, N, prec):
         if self.key != (M, N, prec):
@@ -130,15 +148,27 @@ def _poisson_spectral(rho, bin_size_x, bin_size_y, prec, energy, rho_scale=1.0, 
     return spec
 
 
-def poisson_energy(rho, bin_size_x, bin_size_y, precision):
+def poisson_energy(rho, bin_size_x, bin_size_y, precision, fast=True):
     """Energy (f64[1]) of a normalised density map without the field maps:
     G1 and G2 only (two launches)."""
+    prec = precision_code(precision)
+    if fast and fft_serves(rho, prec):
+        energy = torch.empty(1, dtype=torch.float64, device=rho.device)
+        _poisson_fft(rho, bin_size_x, bin_size_y, 1.0, None, None, None, energy, True)
+        return energy
     energy = torch.zeros(1, dtype=torch.float64, device=rho.device)
-    _poisson_spectral(rho, bin_size_x, bin_size_y, precision_code(precision), energy)
+    _poisson_spectral(rho, bin_size_x, bin_size_y, prec, energy)
     return energy
 
 
-def poisson_solve(rho, bin_size_x, bin_size_y, precision, fast_mode=False, rho_scale=1.0, ws=None):
+def _poisson_fft(rho, bin_size_x, bin_size_y, rho_scale, work, ex, ey, energy, want_energy):
+    """The solve by fast transforms into ex, ey and energy (zero without want_energy)."""
+    dev = rho.device
+    C.poisson_fft(rho, float(rho_scale), float(bin_size_x / bin_size_y), fft_table(rho.size(0), dev),
+                  fft_table(rho.size(1), dev), work, ex, ey, energy, bool(want_energy))
+
+
+def poisson_solve(rho, bin_size_x, bin_size_y, precision, fast_mode=False, rho_scale=1.0, ws=None, fast=True):
     """Field maps and energy of a normalised density map ``rho`` [M, N] (fp32).
 
     Returns (field_map_x, field_map_y, energy_f64[1]); energy is zero when
@@ -146,14 +176,27 @@ def poisson_solve(rho, bin_size_x, bin_size_y, precision, fast_mode=False, rho_s
     rho_scale the map is normalised inside the first GEMM (its alpha): a
     density map and rho_scale = 1 / bin area give the solve of rho.  With a
     PoissonWorkspace ``ws`` nothing is allocated and the results are the
-    workspace's buffers."""
+    workspace's buffers.  fast False: the matrix products, also where the fast
+    transforms would serve the map."""
     prec = precision_code(precision)
     M, N = rho.shape
     dev = rho.device
+    if ws is not None:
+        ws.check(M, N, prec)
+    if fast and fft_serves(rho, prec) and (ws is None or ws.fft_work is not None):
+        if ws is not None:
+            work, ex, ey, energy = ws.fft_work, ws.ex, ws.ey, ws.energy
+        else:
+            work = None
+            ex = torch.empty(M, N, dtype=torch.float32, device=dev)
+            ey = torch.empty(M, N, dtype=torch.float32, device=dev)
+            energy = torch.empty(1, dtype=torch.float64, device=dev)
+        _poisson_fft(rho, bin_size_x, bin_size_y, rho_scale, work, ex, ey, energy, not fast_mode)
+        return ex, ey, energy
     _, chM, shM = transform_matrices(M, prec, dev)
     _, chN, shN = transform_matrices(N, prec, dev)
     if ws is not None:
-        ws.check(M, N, prec)
+        ws.products()
         energy = ws.energy
         C.zero_(energy)
     else:
@@ -180,6 +223,13 @@ def poisson_solve(rho, bin_size_x, bin_size_y, precision, fast_mode=False, rho_s
           chM.as_a(us[1].as_b(dict(lda=M, ldb=M, epilogue=EPI_STORE, alpha=4.0, ldc=N, out_f32=ey)))]
     C.transform_gemm(prec, M, N, M, g4)
     return ex, ey, energy
+
+
+def _fast_solve(precision, deterministic):
+    """Whether a density operator's solve may take the fast transforms: not a
+    split_bf16 one, whose products' own error (up to 1e-3 of the field of a nearly
+    even density) would show between the two."""
+    return precision_code(precision) != 3
 
 
 class ElectricDensityMapFunction(Function):
@@ -434,10 +484,12 @@ class ElectricPotentialFunction(Function):
         if recompute_field:
             # keep only rho; the backward recomputes the field maps
             energy = torch.zeros(1, dtype=torch.float64, device=pos.device) if fast_mode else \
-                poisson_energy(density_map, bin_size_x, bin_size_y, precision)
+                poisson_energy(density_map, bin_size_x, bin_size_y, precision,
+                               _fast_solve(precision, deterministic_flag))
             ctx.field_map_x = ctx.field_map_y = None
         else:
-            ex, ey, energy = poisson_solve(density_map, bin_size_x, bin_size_y, precision, fast_mode)
+            ex, ey, energy = poisson_solve(density_map, bin_size_x, bin_size_y, precision, fast_mode,
+                                           fast=_fast_solve(precision, deterministic_flag))
             ctx.field_map_x = ex
             ctx.field_map_y = ey
         if fast_mode:
@@ -452,7 +504,8 @@ class ElectricPotentialFunction(Function):
         g = grad_pos.reshape(1).to(torch.float32)
         fx, fy = ctx.field_map_x, ctx.field_map_y
         if fx is None:
-            fx, fy, _ = poisson_solve(ctx.density_map, bsx, bsy, ctx.precision, True)
+            fx, fy, _ = poisson_solve(ctx.density_map, bsx, bsy, ctx.precision, True,
+                                      fast=_fast_solve(ctx.precision, ctx.deterministic_flag))
         output = C.electric_force(g, nbx, nby, a, b, c, d, fx.view([-1]), fy.view([-1]),
                                   ctx.pos, sxc, syc, ox, oy, ratio, bcx, bcy, float(xl), float(yl), float(xh),
                                   float(yh), float(bsx), float(bsy), int(nm), int(nf),
@@ -477,10 +530,11 @@ class ElectricPotentialOrderedFunction(Function):
         ctx.density_map = density_map
         if recompute_field:
             energy = torch.zeros(1, dtype=torch.float64, device=pos.device) if fast_mode else \
-                poisson_energy(density_map, bsx, bsy, precision)
+                poisson_energy(density_map, bsx, bsy, precision, _fast_solve(precision, op.deterministic_flag))
             ctx.field_map_x = ctx.field_map_y = None
         else:
-            ex, ey, energy = poisson_solve(density_map, bsx, bsy, precision, fast_mode)
+            ex, ey, energy = poisson_solve(density_map, bsx, bsy, precision, fast_mode,
+                                           fast=_fast_solve(precision, op.deterministic_flag))
             ctx.field_map_x, ctx.field_map_y = ex, ey
         if fast_mode:
             return torch.zeros(1, dtype=pos.dtype, device=pos.device)
@@ -493,7 +547,8 @@ class ElectricPotentialOrderedFunction(Function):
         count = order.numel()
         fx, fy = ctx.field_map_x, ctx.field_map_y
         if fx is None:
-            fx, fy, _ = poisson_solve(ctx.density_map, op.bin_size_x, op.bin_size_y, ctx.precision, True)
+            fx, fy, _ = poisson_solve(ctx.density_map, op.bin_size_x, op.bin_size_y, ctx.precision, True,
+                                      fast=_fast_solve(ctx.precision, op.deterministic_flag))
         g = grad_pos.reshape(1).to(torch.float32)
         force_o = torch.empty(2 * count, dtype=torch.float32, device=g.device)
         C.electric_force_ordered(g, fx.view(-1), fy.view(-1), xy_o, rec4, ratio_o, count, float(op.xl), float(op.yl),

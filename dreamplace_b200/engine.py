@@ -146,8 +146,14 @@ class GPEngine(object):
         self.scratch = torch.empty(ep.num_bins_x * ep.num_bins_y, dtype=torch.int64, device=dev) if self.det else None
         self.prec = precision_code(ep.precision)
         # the Poisson solve's operands and outputs, allocated once: every trial
-        # (eager or captured) of this design solves on its one stream
-        self.poisson_ws = PoissonWorkspace(ep.num_bins_x, ep.num_bins_y, self.prec, dev)
+        # (eager or captured) of this design solves on its one stream.  split_bf16
+        # trials keep the matrix products: the fast transforms' field differs from
+        # theirs by the products' own error (1e-4 of the field of a nearly even
+        # density), which 16 iterations of a 200k-cell design turned into up to 6e-3
+        # of the gradient, and a run's trajectory is to stay what it was (a solve at
+        # 1024^2 takes 67 us instead of 25); dct_precision "fp32" takes the fast
+        # transforms
+        self.poisson_ws = PoissonWorkspace(ep.num_bins_x, ep.num_bins_y, self.prec, dev, fast=self.prec == 0)
         # spatial visiting order of the scattered cells (movable block, then filler
         # block), refreshed every `sort_interval` iterations (refresh_due)
         nm, nf = d.num_movable_nodes, d.num_filler_nodes

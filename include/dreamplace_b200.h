@@ -268,19 +268,46 @@ int dp_transform_gemm(int precision, int M, int N, int K,
  * wv/(wu^2+wv^2)/2, out[2MN:3MN] = 1/(wu^2+wv^2) (0 at [0,0]). */
 int dp_spectral_weights(int M, int N, float wv_scale, float* out, dp_stream_t stream);
 
-/* Reads and clears the tensor-core kernels' device status word (0 = every
- * bounded wait completed; non-zero = a wait expired and the launch returned
- * early).  Synchronises the device. */
+/* ---- the same transforms by fast transforms (power-of-two sides 64 .. 4096) ---
+ * fp32 throughout; each map is read and written once per axis. */
+int dp_fft_supported(int M, int N); /* 1 when both sides are supported */
+/* Table of a side n, written on the host: 4 n floats, exp(-i pi k / 2n) then
+ * exp(-2 pi i k / n) for k < n, interleaved (re, im). */
+int dp_fft_twiddles(int n, float* out_host);
+enum {
+  DP_FFT_DCT2 = 0,       /* 4/(MN) C_M x C_N^T */
+  DP_FFT_IDCT2 = 1,      /* 4 Ch_M x Ch_N^T    */
+  DP_FFT_IDCT_IDXST = 2, /* 4 Ch_M x Sh_N^T    */
+  DP_FFT_IDXST_IDCT = 3  /* 4 Sh_M x Ch_N^T    */
+};
+/* out [M x N] from x [M x N] with work [M x N]; tw_m, tw_n: device copies of
+ * the sides' tables.  All pointers 16-byte aligned. */
+int dp_transform_fft(int kind, const float* x, int M, int N, const float* tw_m, const float* tw_n, float* work,
+                     float* out, dp_stream_t stream);
+/* The Poisson solve of rho * rho_scale (dp_spectral_weights' weights with
+ * wv_scale = bin_size_x / bin_size_y) in three launches: the field maps into ex and ey
+ * [M x N], or interleaved (ex, ey) pairs into exy [M x N x 2], or neither
+ * (all NULL: the energy only), and the energy sum rho * IDCT2(a winv) into
+ * energy[0] (0 without want_energy).  work: 3 M N floats, 16-byte aligned as
+ * every pointer. */
+int dp_poisson_fft(const float* rho, int M, int N, float rho_scale, float wv_scale, const float* tw_m,
+                   const float* tw_n, float* work, float* ex, float* ey, float* exy, double* energy, int want_energy,
+                   dp_stream_t stream);
+
+/* Reads and clears the tensor-core kernels' and the fast transforms' device
+ * status words (0 = every bounded wait completed; non-zero = a wait expired
+ * and the launch returned early).  Synchronises the device. */
 int dp_tc_status(int* status_out);
-/* Bound of every mbarrier wait of the tensor-core kernels, in SM clock cycles
+/* Bound of every mbarrier wait of those kernels, in SM clock cycles
  * (default 4e9, about 2 s); on expiry a kernel records its status word (see
  * dp_tc_status), lets what it issued drain, frees its TMEM and returns.
  * Synchronous; applies to kernels launched afterwards. */
 int dp_tc_set_wait_budget(long long cycles);
 /* Test hook for the bounded waits: while set, the tensor-core kernels' TMA
- * producer issues no copy, so the MMA warp's wait on the first operand stage
- * runs out (status 2) and the kernel returns with nothing in flight; the
- * outputs are then undefined.  Synchronous. */
+ * producer and the fast transforms' row staging issue no copy, so the MMA
+ * warp's wait on the first operand stage, or the wait for the rows, runs out
+ * (status 2) and the kernel returns with nothing in flight; the outputs are
+ * then undefined.  Synchronous. */
 int dp_tc_set_skip_loads(int skip);
 
 /* Operand preparation: out = scale * x, written in the operand format of
