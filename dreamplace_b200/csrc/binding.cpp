@@ -680,6 +680,162 @@ at::Tensor scatter_pairs_to_nodes(at::Tensor vals_o, at::Tensor order, int count
   return out;
 }
 
+// ---------------------------------------------------------------- one trial (dp_trial_*)
+static double* dptr(const at::Tensor& t, int64_t least) {
+  TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kDouble && t.numel() >= least, "expected ", least, " CUDA doubles");
+  return t.data_ptr<double>();
+}
+
+// head: (state_prev, sched_prev, sched_new, hpwl_k, overflow_k, weights_prev, weights_new) or None
+void trial_start(c10::optional<std::vector<at::Tensor>> head, std::vector<double> head_scalars,
+                 c10::optional<at::Tensor> gate, at::Tensor v, at::Tensor g, at::Tensor u, at::Tensor u_new,
+                 at::Tensor v_new, at::Tensor xy_new, at::Tensor state, at::Tensor sx, at::Tensor sy, double xl,
+                 double yl, double xh, double yh, int num_movable, int num_filler,
+                 c10::optional<at::Tensor> inv_order, c10::optional<at::Tensor> xy_order,
+                 std::vector<at::Tensor> zero, at::Tensor cell0, at::Tensor cell1) {
+  const int64_t n2 = v.numel();
+  for (auto* t : {&v, &g, &u, &u_new, &v_new, &xy_new}) {
+    CHECK_CUDA_T(*t); CHECK_CONTIG(*t); CHECK_F32(*t);
+    TORCH_CHECK(t->numel() == n2, "trial_start: size mismatch");
+  }
+  TORCH_CHECK(sx.numel() >= n2 / 2 && sy.numel() >= n2 / 2, "trial_start: size mismatch");
+  TORCH_CHECK(head_scalars.size() == 5 && zero.size() <= 2, "trial_start: bad argument lists");
+  TORCH_CHECK(!head.has_value() || head->size() == 7, "trial_start: the head takes seven tensors");
+  const double* hd[5] = {};
+  const float* w[2] = {};
+  if (head.has_value()) {
+    hd[0] = dptr((*head)[0], DP_NESTEROV_STATE_DOUBLES);
+    hd[1] = dptr((*head)[1], 2);
+    hd[2] = dptr((*head)[2], 2);
+    hd[3] = dptr((*head)[3], 1);
+    hd[4] = dptr((*head)[4], 1);
+    for (int i = 0; i < 2; ++i) {
+      CHECK_F32((*head)[5 + i]);
+      TORCH_CHECK((*head)[5 + i].numel() >= 3, "trial_start: weights hold three floats");
+      w[i] = ptr<float>((*head)[5 + i]);
+    }
+  }
+  if (gate.has_value()) CHECK_I32(*gate);
+  void* z[2] = {};
+  size_t zb[2] = {};
+  for (size_t i = 0; i < zero.size(); ++i) {
+    CHECK_CUDA_T(zero[i]); CHECK_CONTIG(zero[i]);
+    z[i] = zero[i].data_ptr();
+    zb[i] = zero[i].nbytes();
+  }
+  DP_CALL(dp_trial_start(hd[0], hd[1], const_cast<double*>(hd[2]), hd[3], hd[4], w[0], const_cast<float*>(w[1]),
+                         head_scalars[0], head_scalars[1], head_scalars[2], head_scalars[3], head_scalars[4],
+                         gate.has_value() ? ptr<int>(*gate) : nullptr, ptr<float>(v), ptr<float>(g), ptr<float>(u),
+                         ptr<float>(u_new), ptr<float>(v_new), ptr<float>(xy_new),
+                         dptr(state, DP_NESTEROV_STATE_DOUBLES), ptr<float>(sx), ptr<float>(sy), xl, yl, xh, yh,
+                         n2 / 2, num_movable, num_filler, (const int*)ovp(inv_order), (float*)ovp(xy_order), z[0],
+                         zb[0], z[1], zb[1], dptr(cell0, 1), dptr(cell1, 1), cur_stream()));
+}
+
+int trial_wirelength(at::Tensor xy, at::Tensor group_deg, at::Tensor group_base, at::Tensor group_net,
+                     at::Tensor ln_node, at::Tensor ln_offx, at::Tensor ln_offy, c10::optional<at::Tensor> ln_csr,
+                     c10::optional<at::Tensor> net_weights, at::Tensor net_mask, at::Tensor inv_gamma,
+                     at::Tensor wl_f64, at::Tensor grad_node_order, at::Tensor hpwl_mask, at::Tensor hpwl_f64) {
+  CHECK_FLAT(xy); CHECK_F32(xy); CHECK_I32(group_deg); CHECK_I32(group_base); CHECK_I32(group_net);
+  CHECK_I32(ln_node); CHECK_F32(grad_node_order);
+  TORCH_CHECK(group_net.numel() == 32 * group_deg.numel() && group_base.numel() == group_deg.numel(),
+              "trial_wirelength: inconsistent plan");
+  int blocks = 0;
+  DP_CALL(dp_trial_wirelength(ptr<float>(xy), ptr<int>(group_deg), ptr<int>(group_base), ptr<int>(group_net),
+                              group_deg.numel(), ptr<int>(ln_node), ptr<float>(ln_offx), ptr<float>(ln_offy),
+                              (const int*)ovp(ln_csr), (const float*)ovp(net_weights), net_mask.data_ptr<uint8_t>(),
+                              ptr<float>(inv_gamma), dptr(wl_f64, DP_REDUCE_DOUBLES), ptr<float>(grad_node_order),
+                              hpwl_mask.data_ptr<uint8_t>(), dptr(hpwl_f64, DP_REDUCE_DOUBLES), &blocks,
+                              cur_stream()));
+  return blocks;
+}
+
+int trial_density(at::Tensor xy_o, c10::optional<at::Tensor> order, at::Tensor rec4, at::Tensor ratio_o,
+                  int num_first, int count, c10::optional<at::Tensor> init, double xl, double yl, double xh, double yh,
+                  double bsx, double bsy, int nbx, int nby, int deterministic, c10::optional<at::Tensor> scratch2,
+                  at::Tensor out_first, at::Tensor out_all, c10::optional<at::Tensor> all_hi,
+                  c10::optional<at::Tensor> all_lo, double target_area, at::Tensor overflow) {
+  CHECK_FLAT(xy_o); CHECK_F32(xy_o); CHECK_F32(rec4);
+  const int64_t nbins = (int64_t)nbx * nby;
+  if (order.has_value()) {
+    CHECK_I32(*order);
+    TORCH_CHECK(order->numel() >= count, "trial_density: order shorter than count");
+  }
+  TORCH_CHECK(2 * count <= xy_o.numel() && 4 * count <= rec4.numel() && count <= ratio_o.numel(),
+              "trial_density: buffers smaller than count");
+  TORCH_CHECK(out_first.numel() == nbins && out_all.numel() == nbins && (!init.has_value() || init->numel() == nbins),
+              "trial_density: maps are not num_bins_x*num_bins_y");
+  TORCH_CHECK(!deterministic || (scratch2.has_value() && scratch2->scalar_type() == at::kLong &&
+                                 scratch2->numel() >= 2 * nbins),
+              "trial_density: deterministic mode needs two int64 maps");
+  TORCH_CHECK(!all_hi.has_value() || (all_lo.has_value() && all_hi->scalar_type() == at::kBFloat16 &&
+                                      all_lo->scalar_type() == at::kBFloat16 && all_hi->numel() == nbins &&
+                                      all_lo->numel() == nbins),
+              "trial_density: the split operand is two bfloat16 maps");
+  int blocks = 0;
+  DP_CALL(dp_trial_density(ptr<float>(xy_o), (const int*)ovp(order), ptr<float>(rec4), ptr<float>(ratio_o), num_first,
+                           count, (const float*)ovp(init), xl, yl, xh, yh, bsx, bsy, inv_f(bsx), inv_f(bsy), nbx, nby,
+                           deterministic, fraction_bits(xl, yl, xh, yh), (int64_t*)ovp(scratch2),
+                           ptr<float>(out_first), ptr<float>(out_all), ovp(all_hi), ovp(all_lo), target_area,
+                           dptr(overflow, DP_REDUCE_DOUBLES), &blocks, cur_stream()));
+  return blocks;
+}
+
+void trial_force(at::Tensor energy, at::Tensor density_weight, at::Tensor factor_quad, at::Tensor ex, at::Tensor ey,
+                 at::Tensor xy_o, c10::optional<at::Tensor> order, at::Tensor rec4, at::Tensor ratio_o, int count,
+                 double xl, double yl, double bsx, double bsy, int nbx, int nby, double scale, at::Tensor force_o) {
+  CHECK_FLAT(xy_o); CHECK_F32(force_o); CHECK_F32(density_weight); CHECK_F32(factor_quad);
+  TORCH_CHECK(!order.has_value() || order->numel() >= count, "trial_force: order shorter than count");
+  TORCH_CHECK(2 * count <= xy_o.numel() && 4 * count <= rec4.numel() && 2 * count <= force_o.numel() &&
+                  factor_quad.numel() >= 2,
+              "trial_force: buffers smaller than count");
+  TORCH_CHECK(ex.numel() == (int64_t)nbx * nby && ey.numel() == ex.numel(), "trial_force: field map size");
+  DP_CALL(dp_trial_force(dptr(energy, 1), ptr<float>(density_weight), ptr<float>(factor_quad), nbx, nby,
+                         ptr<float>(ex), ptr<float>(ey), ptr<float>(xy_o), (const int*)ovp(order), ptr<float>(rec4),
+                         ptr<float>(ratio_o), count, xl, yl, bsx, bsy, inv_f(bsx), inv_f(bsy), (float)scale,
+                         ptr<float>(force_o), cur_stream()));
+}
+
+int trial_assemble(at::Tensor grad_node_order, at::Tensor node_start, at::Tensor wl_scale, at::Tensor force_o,
+                   at::Tensor inv_order, int num_movable, int num_filler, at::Tensor pws, at::Tensor area,
+                   at::Tensor lambda_, at::Tensor v_new, at::Tensor v, at::Tensor g, at::Tensor g_new,
+                   at::Tensor state, c10::optional<at::Tensor> grad_index) {
+  CHECK_I32(node_start); CHECK_I32(inv_order);
+  int n = v.numel() / 2, blocks = 0;
+  TORCH_CHECK(inv_order.numel() >= n && node_start.numel() >= num_movable + 1 && g_new.numel() == 2 * n,
+              "trial_assemble: size mismatch");
+  DP_CALL(dp_trial_assemble(ptr<float>(grad_node_order), ptr<int>(node_start), ptr<float>(wl_scale),
+                            ptr<float>(force_o), ptr<int>(inv_order), num_movable, num_filler, ptr<float>(pws),
+                            ptr<float>(area), ptr<float>(lambda_), n, ptr<float>(v_new), ptr<float>(v),
+                            ptr<float>(g), ptr<float>(g_new),
+                            dptr(state, DP_NESTEROV_STATE_DOUBLES + 2 * DP_REDUCE_DOUBLES),
+                            (const int*)ovp(grad_index), &blocks, cur_stream()));
+  return blocks;
+}
+
+// out8_host: the device's address of a pinned row (host_pointer), or 0
+void trial_finish(at::Tensor wl, at::Tensor hpwl, int wa_blocks, at::Tensor overflow, int overflow_blocks,
+                  double bin_area, at::Tensor energy, at::Tensor density_weight, at::Tensor factor_quad,
+                  at::Tensor state, int norm_blocks, at::Tensor hpwl_v, at::Tensor overflow_v, at::Tensor obj,
+                  at::Tensor out8, int64_t out8_host) {
+  DP_CALL(dp_trial_finish(dptr(wl, DP_REDUCE_DOUBLES), dptr(hpwl, DP_REDUCE_DOUBLES), wa_blocks,
+                          dptr(overflow, DP_REDUCE_DOUBLES), overflow_blocks, bin_area, dptr(energy, 1),
+                          ptr<float>(density_weight), ptr<float>(factor_quad),
+                          dptr(state, DP_NESTEROV_STATE_DOUBLES + 2 * DP_REDUCE_DOUBLES), norm_blocks,
+                          dptr(hpwl_v, 1), dptr(overflow_v, 2), dptr(obj, 1), dptr(out8, 8),
+                          reinterpret_cast<double*>(out8_host), cur_stream()));
+}
+
+// the device's address of a pinned host tensor, whose owner keeps it alive
+// while kernels or captured graphs write to it
+int64_t host_pointer(at::Tensor t) {
+  TORCH_CHECK(t.is_pinned() && t.is_contiguous(), "host_pointer: a contiguous pinned tensor is needed");
+  void* p = nullptr;
+  cudaError_t e = cudaHostGetDevicePointer(&p, t.data_ptr(), 0);
+  TORCH_CHECK(e == cudaSuccess, "host_pointer: ", cudaGetErrorString(e));
+  return reinterpret_cast<int64_t>(p);
+}
+
 uint64_t launch_count() { return dp_launch_count(); }
 
 // Launches an instantiated CUDA graph (torch.cuda.CUDAGraph.raw_cuda_graph_exec)
@@ -735,6 +891,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("hpwl_forward", &hpwl_forward);
   m.def("move_boundary_forward", &move_boundary_forward);
   m.def("pws_forward", &pws_forward);
+  m.def("trial_start", &trial_start);
+  m.def("trial_wirelength", &trial_wirelength);
+  m.def("trial_density", &trial_density);
+  m.def("trial_force", &trial_force);
+  m.def("trial_assemble", &trial_assemble);
+  m.def("trial_finish", &trial_finish);
+  m.def("host_pointer", &host_pointer);
   m.def("launch_count", &launch_count);
   m.def("graph_launch", &graph_launch);
   m.def("nesterov_init", &nesterov_init);

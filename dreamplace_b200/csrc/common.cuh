@@ -164,4 +164,23 @@ __device__ __forceinline__ long long to_fixed(float v, float scale) {
   return (long long)fmul(v, scale);
 }
 
+// order-preserving float <-> uint32 key: key(a) < key(b) iff a < b; key 0 is
+// below every float, so a zero-filled slot is a valid start for atomicMax
+__device__ __forceinline__ unsigned float_key(float f) {
+  unsigned u = __float_as_uint(f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float key_float(unsigned k) {
+  return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+}
+
+// d objective / d D: the density gradient's scale (see objective_finish_kernel)
+__device__ __forceinline__ float objective_grad_scale(double d, const float* density_weight,
+                                                      const float* factor_quad) {
+  const double lam = (double)factor_quad[0] * (double)density_weight[0];
+  const float quad_c = factor_quad[1];
+  const double dd = quad_c > 0.f ? 1.0 + 2.0 * (double)quad_c * d : 1.0;
+  return (float)(lam * dd);
+}
+
 }  // namespace dpb

@@ -20,6 +20,7 @@
 #include <mutex>
 #include <cuda.h>
 #include <type_traits>
+#include "epilogue.cuh"
 #include "reduce.cuh"
 
 namespace dpb {
@@ -608,16 +609,6 @@ __global__ void clamp_max_kernel(float* map, int n, float vmax) {
     map[i] = fminf(map[i], vmax);
 }
 
-// order-preserving float <-> uint32 key: key(a) < key(b) iff a < b; key 0 is
-// below every float, so a zero-filled slot is a valid start for atomicMax
-__device__ __forceinline__ unsigned float_key(float f) {
-  unsigned u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float key_float(unsigned k) {
-  return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
-}
-
 __global__ void overflow_kernel(const float* __restrict__ map, int n, double target_area,
                                 double* partials, unsigned* maxkey) {
   grid_dep_sync();
@@ -668,51 +659,81 @@ __global__ void first_map_kernel(const long long* __restrict__ fixed, const floa
   block_partial(s, partials);
 }
 
-// fp32 split scatter, second pass: first = init + first (the movable cells
-// were scattered onto a zeroed map), all += first (all held the fillers), and
-// the overflow sum and maximum of first as overflow_kernel does.  float4
-// accesses when the three maps are 16-byte aligned.
-__device__ __forceinline__ void finish_map_bin(float f, float in, float& first_out, float& all_io, double target_area,
-                                               double& s, float& m) {
-  const float d = fadd(in, f);
-  first_out = d;
-  all_io = fadd(d, all_io);
+// Second pass of a scatter into two sums, one bin: first = init + sum0,
+// all = first + sum1 (fp32 sums, each scattered onto a zeroed map) or
+// init + (sum0 + sum1) (fixed point, the int64 sum is exact), with the overflow
+// sum and maximum of first as overflow_kernel does.
+template <typename T>
+__device__ __forceinline__ void finish_map_bin(T f0, T f1, float in, double inv_scale, double target_area, float& d,
+                                               float& all, double& s, float& m) {
+  if constexpr (std::is_same<T, float>::value) {
+    d = fadd(in, f0);
+    all = fadd(d, f1);
+  } else {
+    d = (float)((double)in + (double)f0 * inv_scale);
+    all = (float)((double)in + (double)(f0 + f1) * inv_scale);
+  }
   const double over = (double)d - target_area;
   s += over > 0.0 ? over : 0.0;
   m = fmaxf(m, d);
 }
 
-__global__ void finish_maps_kernel(const float* __restrict__ init, float* __restrict__ first, float* __restrict__ all,
-                                   int n, double target_area, double* partials, unsigned* maxkey,
-                                   const int* __restrict__ gate) {
+template <typename T>
+struct MapSums {
+  const T* sum0;
+  const T* sum1;
+  const float* init;
+  float* first;
+  float* all;
+  __nv_bfloat16* hi;  // optional: all as the split-BF16 operand of the solve's first product
+  __nv_bfloat16* lo;
+  double inv_scale;
+};
+
+// One streaming pass, bound by HBM (four bins a thread and access where the
+// maps are 16-byte aligned).  Writing the solve's bf16 operand here as well
+// saves the pass that read the map again to split it.
+template <typename T>
+__global__ void __launch_bounds__(256) finish_maps_kernel(MapSums<T> a, int n, double target_area, double* partials,
+                                                          unsigned* maxkey, const int* __restrict__ gate) {
   grid_dep_sync();
   if (gate_closed(gate)) return;
   double s = 0.0;
   float m = -INFINITY;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  const bool vec = (((uintptr_t)first | (uintptr_t)all | (uintptr_t)init) & 15) == 0;
+  const bool vec = (((uintptr_t)a.sum0 | (uintptr_t)a.sum1 | (uintptr_t)a.init | (uintptr_t)a.first |
+                     (uintptr_t)a.all | (uintptr_t)a.hi | (uintptr_t)a.lo) & 15) == 0;
   int done = 0;
   if (vec) {
+    struct alignas(16) Four { T v[4]; };
+    struct alignas(16) Four32 { float v[4]; };
+    struct alignas(8) FourBf { __nv_bfloat16 v[4]; };
     const int n4 = n >> 2;
     for (int i = tid; i < n4; i += stride) {
-      const float4 f = reinterpret_cast<const float4*>(first)[i];
-      const float4 in = init ? reinterpret_cast<const float4*>(init)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-      float4 a = reinterpret_cast<const float4*>(all)[i];
-      float4 o;
-      finish_map_bin(f.x, in.x, o.x, a.x, target_area, s, m);
-      finish_map_bin(f.y, in.y, o.y, a.y, target_area, s, m);
-      finish_map_bin(f.z, in.z, o.z, a.z, target_area, s, m);
-      finish_map_bin(f.w, in.w, o.w, a.w, target_area, s, m);
-      reinterpret_cast<float4*>(first)[i] = o;
-      reinterpret_cast<float4*>(all)[i] = a;
+      const Four f0 = reinterpret_cast<const Four*>(a.sum0)[i], f1 = reinterpret_cast<const Four*>(a.sum1)[i];
+      Four32 in = {{0.f, 0.f, 0.f, 0.f}}, d, all;
+      if (a.init) in = reinterpret_cast<const Four32*>(a.init)[i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        finish_map_bin(f0.v[j], f1.v[j], in.v[j], a.inv_scale, target_area, d.v[j], all.v[j], s, m);
+      reinterpret_cast<Four32*>(a.first)[i] = d;
+      reinterpret_cast<Four32*>(a.all)[i] = all;
+      if (a.hi) {
+        FourBf h, l;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) store_operand(kFmtSplit, all.v[j], j, nullptr, h.v, l.v);
+        reinterpret_cast<FourBf*>(a.hi)[i] = h;
+        reinterpret_cast<FourBf*>(a.lo)[i] = l;
+      }
     }
     done = n4 << 2;
   }
   for (int i = done + tid; i < n; i += stride) {
-    float o, a = all[i];
-    finish_map_bin(first[i], init ? init[i] : 0.f, o, a, target_area, s, m);
-    first[i] = o;
-    all[i] = a;
+    float d, all;
+    finish_map_bin(a.sum0[i], a.sum1[i], a.init ? a.init[i] : 0.f, a.inv_scale, target_area, d, all, s, m);
+    a.first[i] = d;
+    a.all[i] = all;
+    if (a.hi) store_operand(kFmtSplit, all, i, nullptr, a.hi, a.lo);
   }
   if (!partials) return;  // uniform: no overflow wanted
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -1085,13 +1106,59 @@ extern "C" int dp_density_map_ordered_split(const float* xy_o, const int* order,
   rc = scatter_ranges(o, rg, 0, 0);
   if (rc) return rc;
   if (overflow_out) cudaMemsetAsync(maxslot, 0, sizeof(double), o.s);
-  launch_kernel(finish_maps_kernel, blocks, 256, 0, o.s, init, out_first, out_all, nbins, target_area,
-                                             overflow_out ? overflow_out + 3 : nullptr, maxslot, trial_gate());
+  const MapSums<float> sums = {out_first, out_all, init, out_first, out_all, nullptr, nullptr, 0.0};
+  launch_kernel(finish_maps_kernel<float>, blocks, 256, 0, o.s, sums, nbins, target_area,
+                overflow_out ? overflow_out + 3 : nullptr, maxslot, trial_gate());
   rc = check_launch("dp_density_map_ordered_split first map");
   if (rc || !overflow_out) return rc;
   launch_kernel(overflow_finish_kernel, 1, kReduceThreads, 0, o.s, overflow_out, maxslot, bin_area, nullptr,
                                                         overflow_out + 3, blocks);
   return check_launch("dp_density_map_ordered_split overflow");
+}
+
+// The split scatter inside a trial: both ranges in one launch (the fillers'
+// blocks fill the movable cells' last wave, also in fixed point, where the two
+// sums have a map each), onto sums that dp_trial_start zeroed; the overflow's
+// partials stay for dp_trial_finish.
+extern "C" int dp_trial_density(const float* xy_o, const int* order, const float* rec4, const float* ratio_o,
+                                int num_first, int count, const float* init, float xl, float yl, float xh, float yh,
+                                float bsx, float bsy, float ibx, float iby, int nbx, int nby, int deterministic,
+                                int fraction_bits, int64_t* scratch2, float* out_first, float* out_all, void* all_hi,
+                                void* all_lo, double target_area, double* overflow, int* overflow_blocks,
+                                dp_stream_t stream) {
+  OrderedScatter o;
+  int rc = ordered_setup("dp_trial_density", xy_o, order, rec4, ratio_o, count, xl, yl, bsx, bsy, ibx, iby, nbx, nby,
+                         deterministic, fraction_bits, scratch2, stream, o);
+  if (rc) return rc;
+  DP_REQUIRE(out_first && out_all && out_first != out_all && overflow && overflow_blocks, "dp_trial_density: bad outputs");
+  DP_REQUIRE(num_first >= 0 && num_first <= count, "dp_trial_density: bad num_first");
+  DP_REQUIRE(!all_hi == !all_lo, "dp_trial_density: the split operand needs both halves");
+  const int nbins = nbx * nby;
+  WsRanges rg;
+  memset(&rg, 0, sizeof(rg));
+  rg.b1 = num_first;
+  rg.b2 = count;
+  rg.map0_f32 = out_first;
+  rg.map1_f32 = out_all;
+  rg.map0_fx = reinterpret_cast<unsigned long long*>(scratch2);
+  rg.map1_fx = rg.map0_fx + (deterministic ? nbins : 0);
+  rc = scatter_ranges(o, rg, deterministic, fraction_bits);
+  if (rc) return rc;
+  const int blocks = grid_for(nbins, 256, 4);
+  *overflow_blocks = blocks;
+  unsigned* maxslot = reinterpret_cast<unsigned*>(overflow + 2);
+  __nv_bfloat16 *hi = (__nv_bfloat16*)all_hi, *lo = (__nv_bfloat16*)all_lo;
+  if (deterministic) {
+    const MapSums<long long> sums = {(const long long*)scratch2, (const long long*)scratch2 + nbins, init, out_first,
+                                     out_all, hi, lo, ldexp(1.0, -fraction_bits)};
+    launch_kernel(finish_maps_kernel<long long>, blocks, 256, 0, o.s, sums, nbins, target_area, overflow + 3, maxslot,
+                  trial_gate());
+  } else {
+    const MapSums<float> sums = {out_first, out_all, init, out_first, out_all, hi, lo, 0.0};
+    launch_kernel(finish_maps_kernel<float>, blocks, 256, 0, o.s, sums, nbins, target_area, overflow + 3, maxslot,
+                  trial_gate());
+  }
+  return check_launch("dp_trial_density finish");
 }
 
 // ---------------------------------------------------------------- allocation-free variant

@@ -65,14 +65,21 @@ constexpr int kForceWin = 3;  // almost every stretched cell covers at most 3 x 
 // node order read through `order`); the force pair is written in order
 // space, force_o[idx] = scale * grad * ratio * sum(px py E), for the gradient
 // assembly kernel to pick up per node.
+struct ForceScale {
+  const float* grad_pos;  // the scale itself, or nullptr: d objective / d D from the words below
+  const double* energy;
+  const float* density_weight;
+  const float* factor_quad;
+};
+
 __global__ void __launch_bounds__(256) electric_force_records_kernel(
-    const float* __restrict__ grad_pos, int nbx, int nby, const float* __restrict__ ex, const float* __restrict__ ey,
+    ForceScale fs, int nbx, int nby, const float* __restrict__ ex, const float* __restrict__ ey,
     const float2* __restrict__ xy_o, const int* __restrict__ order, const float4* __restrict__ rec4,
     const float* __restrict__ ratio_o, int count, float xl, float yl, float bsx, float bsy, float ibx, float iby,
     float scale, float2* __restrict__ force_o, const int* __restrict__ gate) {
   grid_dep_sync();
   if (gate_closed(gate)) return;
-  const float g = grad_pos[0];
+  const float g = fs.grad_pos ? fs.grad_pos[0] : objective_grad_scale(fs.energy[0], fs.density_weight, fs.factor_quad);
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
     const float4 r4 = __ldcs(rec4 + idx);
     const float2 p = order ? __ldg(xy_o + __ldg(order + idx)) : __ldg(xy_o + idx);
@@ -127,20 +134,42 @@ __global__ void __launch_bounds__(256) electric_force_records_kernel(
 
 using namespace dpb;
 
-extern "C" int dp_electric_force_ordered(const float* grad_pos, int nbx, int nby, const float* ex, const float* ey,
+static int force_ordered(const ForceScale& fs, int nbx, int nby, const float* ex, const float* ey,
                                          const float* xy_o, const int* order, const float* rec4,
                                          const float* ratio_o,
                                          int count, float xl, float yl, float bsx, float bsy, float ibx, float iby,
                                          float scale, float* force_o, dp_stream_t stream) {
-  DP_REQUIRE(grad_pos && ex && ey && xy_o && rec4 && ratio_o && force_o,
+  DP_REQUIRE(ex && ey && xy_o && rec4 && ratio_o && force_o,
              "dp_electric_force_ordered: null pointer argument");
   DP_REQUIRE(((uintptr_t)xy_o & 7) == 0 && ((uintptr_t)rec4 & 15) == 0 && ((uintptr_t)force_o & 7) == 0,
              "dp_electric_force_ordered: misaligned xy_o / rec4 / force_o");
   if (count == 0) return DP_OK;
   launch_kernel(electric_force_records_kernel, grid_for(count, 256, 16), 256, 0, as_stream(stream), 
-      grad_pos, nbx, nby, ex, ey, reinterpret_cast<const float2*>(xy_o), order, reinterpret_cast<const float4*>(rec4),
+      fs, nbx, nby, ex, ey, reinterpret_cast<const float2*>(xy_o), order, reinterpret_cast<const float4*>(rec4),
       ratio_o, count, xl, yl, bsx, bsy, ibx, iby, scale, reinterpret_cast<float2*>(force_o), trial_gate());
   return check_launch("dp_electric_force_ordered");
+}
+
+extern "C" int dp_electric_force_ordered(const float* grad_pos, int nbx, int nby, const float* ex, const float* ey,
+                                         const float* xy_o, const int* order, const float* rec4,
+                                         const float* ratio_o,
+                                         int count, float xl, float yl, float bsx, float bsy, float ibx, float iby,
+                                         float scale, float* force_o, dp_stream_t stream) {
+  DP_REQUIRE(grad_pos, "dp_electric_force_ordered: null pointer argument");
+  const ForceScale fs = {grad_pos, nullptr, nullptr, nullptr};
+  return force_ordered(fs, nbx, nby, ex, ey, xy_o, order, rec4, ratio_o, count, xl, yl, bsx, bsy, ibx, iby, scale,
+                       force_o, stream);
+}
+
+extern "C" int dp_trial_force(const double* energy, const float* density_weight, const float* factor_quad, int nbx, int nby, const float* ex, const float* ey,
+                                         const float* xy_o, const int* order, const float* rec4,
+                                         const float* ratio_o,
+                                         int count, float xl, float yl, float bsx, float bsy, float ibx, float iby,
+                                         float scale, float* force_o, dp_stream_t stream) {
+  DP_REQUIRE(energy && density_weight && factor_quad, "dp_trial_force: null pointer argument");
+  const ForceScale fs = {nullptr, energy, density_weight, factor_quad};
+  return force_ordered(fs, nbx, nby, ex, ey, xy_o, order, rec4, ratio_o, count, xl, yl, bsx, bsy, ibx, iby, scale,
+                       force_o, stream);
 }
 
 extern "C" int dp_electric_force(const float* grad_pos, int nbx, int nby, const float* ex,

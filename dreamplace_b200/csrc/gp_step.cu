@@ -56,36 +56,52 @@ enum {
 // u' = v - alpha g; v' = u' + coef (u' - u); v' clamped into the die for
 // movable and filler nodes (move_boundary semantics); one thread per node
 // also writes the interleaved copy xy' used by the gather kernels.
-__global__ void nesterov_trial_kernel(const float* __restrict__ v, const float* __restrict__ g,
-                                      const float* __restrict__ u, float* __restrict__ u_new,
-                                      float* __restrict__ v_new, float2* __restrict__ xy_new,
-                                      const double* __restrict__ st, const float* __restrict__ sx,
-                                      const float* __restrict__ sy, float xl, float yl, float xh, float yh,
-                                      int num_nodes, int num_movable, int num_filler,
-                                      const int* __restrict__ inv_order, float2* __restrict__ xy_o,
-                                      const int* __restrict__ gate) {
-  grid_dep_sync();
-  if (gate_closed(gate)) return;
-  const float alpha = (float)st[NS_ALPHA];
-  const float coef = (float)st[NS_COEF];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < num_nodes; i += gridDim.x * blockDim.x) {
-    const int j = i + num_nodes;
+struct TrialPoint {
+  const float* v;
+  const float* g;
+  const float* u;
+  float* u_new;
+  float* v_new;
+  float2* xy_new;
+  const double* st;
+  const float* sx;
+  const float* sy;
+  float xl, yl, xh, yh;
+  int num_nodes, num_movable, num_filler;
+  const int* inv_order;
+  float2* xy_o;
+};
+
+__device__ __forceinline__ void trial_point(const TrialPoint& p, float alpha, float coef, int tid, int stride) {
+  const float* __restrict__ v = p.v;
+  const float* __restrict__ g = p.g;
+  const float* __restrict__ u = p.u;
+  for (int i = tid; i < p.num_nodes; i += stride) {
+    const int j = i + p.num_nodes;
     const float ux = fsub(v[i], fmul(alpha, g[i]));
     const float uy = fsub(v[j], fmul(alpha, g[j]));
     float vx = fadd(ux, fmul(coef, fsub(ux, u[i])));
     float vy = fadd(uy, fmul(coef, fsub(uy, u[j])));
-    if (i < num_movable || i >= num_nodes - num_filler) {
-      vx = fminf(fmaxf(vx, xl), fsub(xh, sx[i]));
-      vy = fminf(fmaxf(vy, yl), fsub(yh, sy[i]));
+    const bool cell = i < p.num_movable || i >= p.num_nodes - p.num_filler;
+    if (cell) {
+      vx = fminf(fmaxf(vx, p.xl), fsub(p.xh, p.sx[i]));
+      vy = fminf(fmaxf(vy, p.yl), fsub(p.yh, p.sy[i]));
     }
-    u_new[i] = ux;
-    u_new[j] = uy;
-    v_new[i] = vx;
-    v_new[j] = vy;
-    if (xy_new) xy_new[i] = make_float2(vx, vy);
+    p.u_new[i] = ux;
+    p.u_new[j] = uy;
+    p.v_new[i] = vx;
+    p.v_new[j] = vy;
+    if (p.xy_new) p.xy_new[i] = make_float2(vx, vy);
     // the scattered cells' positions also land in visiting order
-    if (xy_o && (i < num_movable || i >= num_nodes - num_filler)) xy_o[inv_order[i]] = make_float2(vx, vy);
+    if (p.xy_o && cell) p.xy_o[p.inv_order[i]] = make_float2(vx, vy);
   }
+}
+
+__global__ void nesterov_trial_kernel(TrialPoint p, const int* __restrict__ gate) {
+  grid_dep_sync();
+  if (gate_closed(gate)) return;
+  trial_point(p, (float)p.st[NS_ALPHA], (float)p.st[NS_COEF], blockIdx.x * blockDim.x + threadIdx.x,
+              gridDim.x * blockDim.x);
 }
 
 __global__ void pack_xy_kernel(const float* __restrict__ v, float2* __restrict__ xy, int num_nodes) {
@@ -223,11 +239,7 @@ __global__ void __launch_bounds__(kAsmThreads, 4) assemble_precondition_kernel(
   block_partial2(dv, dg, partials);
 }
 
-__global__ void nesterov_finish_kernel(double* st, const double* partials, int count) {
-  grid_dep_sync();
-  double dv = finish_sum(partials, count);
-  double dg = finish_sum(partials + count, count);
-  if (threadIdx.x != 0) return;
+__device__ __forceinline__ void nesterov_test(double* st, double dv, double dg) {
   st[NS_ACC_DV] = dv;
   st[NS_ACC_DG] = dg;
   double an = sqrt(dv / dg);
@@ -235,6 +247,14 @@ __global__ void nesterov_finish_kernel(double* st, const double* partials, int c
   st[NS_ALPHA_NEW] = an;
   st[NS_ACCEPT] = accept;
   st[NS_ALPHA] = an;  // the reference copies alpha_{k+1} into alpha_k after every trial
+}
+
+__global__ void nesterov_finish_kernel(double* st, const double* partials, int count) {
+  grid_dep_sync();
+  double dv = finish_sum(partials, count);
+  double dg = finish_sum(partials + count, count);
+  if (threadIdx.x != 0) return;
+  nesterov_test(st, dv, dg);
 }
 
 __global__ void nesterov_init_kernel(double* st, double alpha) {
@@ -251,16 +271,84 @@ __global__ void nesterov_init_kernel(double* st, double alpha) {
 // penalty (c > 0) and lambda_eff = density_factor * density_weight; the density
 // gradient's scale (d objective / d D) goes to grad_scale for the force kernel
 // (dreamplace/PlaceObj.py:293-320).
+__device__ __forceinline__ double objective_value(double wl, double d, const float* density_weight,
+                                                  const float* factor_quad) {
+  const double lam = (double)factor_quad[0] * (double)density_weight[0];
+  const float quad_c = factor_quad[1];
+  const double dp = quad_c > 0.f ? d * (1.0 + (double)quad_c * d) : d;
+  return wl + lam * dp;
+}
+
 __global__ void objective_finish_kernel(const double* wl, const double* energy, const float* density_weight,
                                         const float* factor_quad, double* obj, float* grad_scale) {
   grid_dep_sync();
-  const float density_factor = factor_quad[0], quad_c = factor_quad[1];
-  double lam = (double)density_factor * (double)density_weight[0];
-  double d = energy[0];
-  double dp = quad_c > 0.f ? d * (1.0 + (double)quad_c * d) : d;
-  if (obj) obj[0] = wl[0] + lam * dp;
-  double dd = quad_c > 0.f ? 1.0 + 2.0 * (double)quad_c * d : 1.0;
-  if (grad_scale) grad_scale[0] = (float)(lam * dd);
+  if (obj) obj[0] = objective_value(wl[0], energy[0], density_weight, factor_quad);
+  if (grad_scale) grad_scale[0] = objective_grad_scale(energy[0], density_weight, factor_quad);
+}
+
+// The end of a trial in one block: the fixed-order sums of the WA, HPWL,
+// overflow and step-size partials (the order of finish_sum for each, so every
+// total is what its own finisher gives), the objective, the Nesterov test and
+// the metrics row, which is also written to the host's pinned copy.  As
+// separate nodes these were five one-block kernels and a copy.
+struct TrialFinish {
+  double* wl;      // [0] total, [1..] partials
+  double* hpwl;
+  int wa_blocks;
+  double* ovf;     // [0] overflow, [1] largest density, [2] its key, [3..] partials
+  int ovf_blocks;
+  double bin_area;
+  const double* energy;
+  const float* density_weight;
+  const float* factor_quad;
+  double* st;      // Nesterov scalars, then 2 x norm_blocks partials
+  int norm_blocks;
+  const double* hpwl_v;  // metrics of v_k
+  const double* ovf_v;
+  double* obj;
+  double* out;
+  double* out_host;
+};
+
+__global__ void __launch_bounds__(kReduceThreads) trial_finish_kernel(TrialFinish a) {
+  grid_dep_sync();
+  __shared__ double sh[5][kReduceThreads / 32];
+  const double* src[5] = {a.wl + 1, a.hpwl + 1, a.ovf + 3, a.st + DP_NESTEROV_STATE_DOUBLES,
+                          a.st + DP_NESTEROV_STATE_DOUBLES + a.norm_blocks};
+  const int cnt[5] = {a.wa_blocks, a.wa_blocks, a.ovf_blocks, a.norm_blocks, a.norm_blocks};
+  double v[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    v[k] = 0.0;
+    for (int i = threadIdx.x; i < cnt[k]; i += kReduceThreads) v[k] += src[k][i];
+  }
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    v[k] = warp_sum(v[k]);
+    if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = v[k];
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double r[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    r[k] = 0.0;
+    for (int w = 0; w < kReduceThreads / 32; ++w) r[k] += sh[k][w];
+  }
+  a.wl[0] = r[0];
+  a.hpwl[0] = r[1];
+  a.ovf[0] = r[2];
+  a.ovf[1] = (double)key_float(*reinterpret_cast<const unsigned*>(a.ovf + 2)) / a.bin_area;
+  const double e = a.energy[0];
+  const double obj = objective_value(r[0], e, a.density_weight, a.factor_quad);
+  a.obj[0] = obj;
+  nesterov_test(a.st, r[3], r[4]);
+  const double m[8] = {a.hpwl_v[0], a.ovf_v[0], a.ovf_v[1], a.st[NS_ACCEPT], a.st[NS_ALPHA], obj, r[0], e};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    a.out[i] = m[i];
+    if (a.out_host) a.out_host[i] = m[i];
+  }
 }
 
 // the metrics a trial's host read-back needs, gathered into one 8-double row:
@@ -290,6 +378,24 @@ extern "C" int dp_trial_metrics(const double* hpwl, const double* overflow2, con
   return check_launch("dp_trial_metrics");
 }
 
+extern "C" int dp_trial_finish(double* wl, double* hpwl, int wa_blocks, double* overflow, int overflow_blocks,
+                               double bin_area, const double* energy, const float* density_weight,
+                               const float* factor_quad, double* state, int norm_blocks, const double* hpwl_v,
+                               const double* overflow_v, double* obj, double* out8, double* out8_host,
+                               dp_stream_t stream) {
+  DP_REQUIRE(wl && hpwl && overflow && energy && density_weight && factor_quad && state && hpwl_v && overflow_v &&
+                 obj && out8,
+             "dp_trial_finish: null pointer");
+  DP_REQUIRE(wa_blocks >= 0 && wa_blocks <= kMaxReduceBlocks && overflow_blocks >= 0 &&
+                 overflow_blocks <= DP_REDUCE_DOUBLES - 3 && norm_blocks >= 0 && norm_blocks <= DP_REDUCE_DOUBLES &&
+                 bin_area > 0.0,
+             "dp_trial_finish: bad counts");
+  const TrialFinish a = {wl, hpwl, wa_blocks, overflow, overflow_blocks, bin_area, energy, density_weight, factor_quad,
+                         state, norm_blocks, hpwl_v, overflow_v, obj, out8, out8_host};
+  launch_kernel(trial_finish_kernel, 1, kReduceThreads, 0, as_stream(stream), a);
+  return check_launch("dp_trial_finish");
+}
+
 extern "C" int dp_objective_finish(const double* wl, const double* energy, const float* density_weight,
                                    const float* factor_quad, double* obj, float* grad_scale, dp_stream_t stream) {
   DP_REQUIRE(energy && density_weight && factor_quad && (obj || grad_scale) && (!obj || wl),
@@ -313,9 +419,9 @@ extern "C" int dp_nesterov_trial(const float* v, const float* g, const float* u,
              "dp_nesterov_trial: xy_new / xy_order must be 8-byte aligned");
   DP_REQUIRE(!xy_order || inv_order, "dp_nesterov_trial: xy_order needs inv_order");
   if (num_nodes == 0) return DP_OK;
-  launch_kernel(nesterov_trial_kernel, grid_for(num_nodes, 256, 8), 256, 0, as_stream(stream), 
-      v, g, u, u_new, v_new, reinterpret_cast<float2*>(xy_new), state, sx, sy, xl, yl, xh, yh, num_nodes, num_movable,
-      num_filler, inv_order, reinterpret_cast<float2*>(xy_order), trial_gate());
+  const TrialPoint p = {v, g, u, u_new, v_new, reinterpret_cast<float2*>(xy_new), state, sx, sy, xl, yl, xh, yh,
+                        num_nodes, num_movable, num_filler, inv_order, reinterpret_cast<float2*>(xy_order)};
+  launch_kernel(nesterov_trial_kernel, grid_for(num_nodes, 256, 8), 256, 0, as_stream(stream), p, trial_gate());
   return check_launch("dp_nesterov_trial");
 }
 
@@ -356,41 +462,111 @@ extern "C" int dp_precondition_step_size(float* g_new, const float* g, const flo
 //    10^((ovf_k / total_area - 0.1) * 20 / 9 - 1), rounded to float, and its
 //    reciprocal (the WA kernel's scalar).
 // sched = {k, hpwl_{k-1}}; weights = {lambda, gamma, 1 / gamma}.
-__global__ void iteration_head_kernel(const double* __restrict__ st_prev, double* __restrict__ st_new,
-                                      const double* __restrict__ sched_prev, double* __restrict__ sched_new,
-                                      const double* __restrict__ hpwl_k, const double* __restrict__ ovf_k,
-                                      const float* __restrict__ w_prev, float* __restrict__ w_new, double base_gamma,
-                                      double total_area, double ref_hpwl, double lower, double upper, int* gate) {
+namespace dpb {
+
+struct HeadArgs {
+  const double* st_prev;
+  double* st_new;
+  const double* sched_prev;
+  double* sched_new;
+  const double* hpwl_k;
+  const double* ovf_k;
+  const float* w_prev;
+  float* w_new;
+  double base_gamma, total_area, ref_hpwl, lower, upper;
+};
+
+// a_{k+1} of the Nesterov sequence
+__device__ __forceinline__ double momentum_next(double a) { return (1.0 + sqrt(4.0 * a * a + 1.0)) / 2.0; }
+
+__device__ __forceinline__ void iteration_head(const HeadArgs& h) {
+  for (int i = 0; i < DP_NESTEROV_STATE_DOUBLES; ++i) h.st_new[i] = h.st_prev[i];
+  const double a = h.st_new[NS_A_NEXT];
+  h.st_new[NS_A] = a;
+  const double an = momentum_next(a);
+  h.st_new[NS_A_NEXT] = an;
+  h.st_new[NS_COEF] = (a - 1.0) / an;
+  const double f = h.sched_prev[0] + 1.0;
+  const double hp = h.hpwl_k[0];
+  float lam = h.w_prev[0];
+  if (f > 1.0) {
+    const double delta = hp - h.sched_prev[1];
+    double mu;
+    if (delta < 0.0)
+      mu = h.upper * fmax(pow(0.9999, f), 0.98);
+    else
+      mu = h.upper * fmin(fmax(pow(h.upper, -delta / h.ref_hpwl), h.lower), h.upper);
+    lam = fmul(lam, (float)mu);
+  }
+  h.sched_new[0] = f;
+  h.sched_new[1] = hp;
+  const double t = (h.ovf_k[0] / h.total_area - 0.1) * 20.0 / 9.0 - 1.0;
+  const float gamma = (float)(h.base_gamma * pow(10.0, t));
+  h.w_new[0] = lam;
+  h.w_new[1] = gamma;
+  h.w_new[2] = __fdiv_rn(1.0f, gamma);
+}
+
+__global__ void iteration_head_kernel(HeadArgs h, int* gate) {
   grid_dep_sync();
   // the previous trial was rejected: this iteration was enqueued ahead and is
   // void; its gated kernels return at once
-  if (gate) *gate = st_prev[NS_ACCEPT] == 0.0 ? 1 : 0;
-  for (int i = 0; i < DP_NESTEROV_STATE_DOUBLES; ++i) st_new[i] = st_prev[i];
-  const double a = st_new[NS_A_NEXT];
-  st_new[NS_A] = a;
-  const double an = (1.0 + sqrt(4.0 * a * a + 1.0)) / 2.0;
-  st_new[NS_A_NEXT] = an;
-  st_new[NS_COEF] = (a - 1.0) / an;
-  const double f = sched_prev[0] + 1.0;
-  const double hp = hpwl_k[0];
-  float lam = w_prev[0];
-  if (f > 1.0) {
-    const double delta = hp - sched_prev[1];
-    double mu;
-    if (delta < 0.0)
-      mu = upper * fmax(pow(0.9999, f), 0.98);
-    else
-      mu = upper * fmin(fmax(pow(upper, -delta / ref_hpwl), lower), upper);
-    lam = fmul(lam, (float)mu);
-  }
-  sched_new[0] = f;
-  sched_new[1] = hp;
-  const double t = (ovf_k[0] / total_area - 0.1) * 20.0 / 9.0 - 1.0;
-  const float gamma = (float)(base_gamma * pow(10.0, t));
-  w_new[0] = lam;
-  w_new[1] = gamma;
-  w_new[2] = __fdiv_rn(1.0f, gamma);
+  if (gate) *gate = h.st_prev[NS_ACCEPT] == 0.0 ? 1 : 0;
+  iteration_head(h);
 }
+
+// The start of a trial in one launch: the between-iteration work (head, when
+// h.st_prev is given) or the gate reset, the trial point, and the zeroing of
+// what the trial's later kernels add into (the density sums, the energy, the
+// largest density).  A trial of a small design is bound by the number of its
+// graph nodes: as separate nodes these were the head, the trial point and four
+// memsets, each of which also broke the programmatic overlap of the kernels
+// around it (~2 us a node; an iteration of 10k cells 148 -> 99 us, of 200k
+// 208 -> 166, of 2.1M 1% less, all with the finishers folded as well).  The first block does the head alone -- its two
+// pow() calls take longer than another block's share of the nodes -- and every
+// other block forms alpha and the momentum coefficient from the previous
+// state itself, so none waits for it.
+struct TrialZero {
+  uint32_t* a[2];          // 4-byte words, 16-byte aligned
+  long long words[2];
+  double* cell[2];
+};
+
+__global__ void __launch_bounds__(256) trial_start_kernel(HeadArgs h, int* gate, TrialZero z, TrialPoint p) {
+  grid_dep_sync();
+  const bool head = h.st_prev != nullptr;
+  const bool closed = head && gate && h.st_prev[NS_ACCEPT] == 0.0;
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) {
+      if (gate) *gate = closed ? 1 : 0;
+      if (head) iteration_head(h);
+      for (int i = 0; i < 2; ++i)
+        if (z.cell[i] && !closed) *z.cell[i] = 0.0;
+    }
+    return;
+  }
+  if (closed) return;
+  float alpha, coef;
+  if (head) {
+    const double a = h.st_prev[NS_A_NEXT];
+    alpha = (float)h.st_prev[NS_ALPHA];
+    coef = (float)((a - 1.0) / momentum_next(a));
+  } else {
+    alpha = (float)p.st[NS_ALPHA];
+    coef = (float)p.st[NS_COEF];
+  }
+  const int tid = (blockIdx.x - 1) * blockDim.x + threadIdx.x, stride = (gridDim.x - 1) * blockDim.x;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const long long n4 = z.words[r] >> 2;
+    for (long long i = tid; i < n4; i += stride) reinterpret_cast<uint4*>(z.a[r])[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (tid < (z.words[r] & 3)) z.a[r][4 * n4 + tid] = 0u;
+  }
+  trial_point(p, alpha, coef, tid, stride);
+}
+
+}  // namespace dpb
+using namespace dpb;
 
 extern "C" int dp_iteration_head(const double* state_prev, double* state_new, const double* sched_prev,
                                  double* sched_new, const double* hpwl_k, const double* overflow_k,
@@ -402,10 +578,39 @@ extern "C" int dp_iteration_head(const double* state_prev, double* state_new, co
   DP_REQUIRE(state_prev != state_new && sched_prev != sched_new && weights_prev != weights_new,
              "dp_iteration_head: the previous and the new iteration need separate buffers");
   DP_REQUIRE(total_area > 0.0 && ref_hpwl > 0.0, "dp_iteration_head: total_area and ref_hpwl must be positive");
-  launch_kernel(iteration_head_kernel, 1, 1, 0, as_stream(stream), state_prev, state_new, sched_prev, sched_new, hpwl_k,
-                                                        overflow_k, weights_prev, weights_new, base_gamma,
-                                                        total_area, ref_hpwl, lower, upper, gate);
+  const HeadArgs h = {state_prev, state_new, sched_prev, sched_new, hpwl_k, overflow_k, weights_prev, weights_new,
+                      base_gamma, total_area, ref_hpwl, lower, upper};
+  launch_kernel(iteration_head_kernel, 1, 1, 0, as_stream(stream), h, gate);
   return check_launch("dp_iteration_head");
+}
+
+extern "C" int dp_trial_start(const double* state_prev, const double* sched_prev, double* sched_new,
+                              const double* hpwl_k, const double* overflow_k, const float* weights_prev,
+                              float* weights_new, double base_gamma, double total_area, double ref_hpwl, double lower,
+                              double upper, int* gate, const float* v, const float* g, const float* u, float* u_new,
+                              float* v_new, float* xy_new, double* state, const float* sx, const float* sy, float xl,
+                              float yl, float xh, float yh, int num_nodes, int num_movable, int num_filler,
+                              const int* inv_order, float* xy_order, void* zero0, size_t zero0_bytes, void* zero1,
+                              size_t zero1_bytes, double* zero_cell0, double* zero_cell1, dp_stream_t stream) {
+  DP_REQUIRE(v && g && u && u_new && v_new && state && sx && sy && num_nodes > 0, "dp_trial_start: bad arguments");
+  DP_REQUIRE(!state_prev || (sched_prev && sched_new && hpwl_k && overflow_k && weights_prev && weights_new &&
+                             state_prev != state && sched_prev != sched_new && weights_prev != weights_new &&
+                             total_area > 0.0 && ref_hpwl > 0.0),
+             "dp_trial_start: bad arguments of the iteration head");
+  DP_REQUIRE(((uintptr_t)xy_new & 7) == 0 && ((uintptr_t)xy_order & 7) == 0,
+             "dp_trial_start: xy_new / xy_order must be 8-byte aligned");
+  DP_REQUIRE(!xy_order || inv_order, "dp_trial_start: xy_order needs inv_order");
+  DP_REQUIRE((((uintptr_t)zero0 | (uintptr_t)zero1) & 15) == 0 && ((zero0_bytes | zero1_bytes) & 3) == 0 &&
+                 (zero0 || !zero0_bytes) && (zero1 || !zero1_bytes),
+             "dp_trial_start: the zeroed ranges must be 16-byte aligned whole words");
+  HeadArgs h = {state_prev, state, sched_prev, sched_new, hpwl_k, overflow_k, weights_prev, weights_new,
+                base_gamma, total_area, ref_hpwl, lower, upper};
+  TrialZero z = {{(uint32_t*)zero0, (uint32_t*)zero1}, {(long long)zero0_bytes / 4, (long long)zero1_bytes / 4},
+                 {zero_cell0, zero_cell1}};
+  const TrialPoint p = {v, g, u, u_new, v_new, reinterpret_cast<float2*>(xy_new), state, sx, sy, xl, yl, xh, yh,
+                        num_nodes, num_movable, num_filler, inv_order, reinterpret_cast<float2*>(xy_order)};
+  launch_kernel(trial_start_kernel, 1 + grid_for(num_nodes, 256, 8), 256, 0, as_stream(stream), h, gate, z, p);
+  return check_launch("dp_trial_start");
 }
 
 // ============================================================== warp reductions, pin sums
@@ -461,19 +666,18 @@ extern "C" int dp_node_pin_sum(const float* grad_node_order, int num_slots, cons
   return dpb::check_launch("dp_node_pin_sum");
 }
 
-extern "C" int dp_assemble_precondition_step(const float* grad_node_order, const int* node_start,
+static int launch_assemble(const float* grad_node_order, const int* node_start,
                                              const float* wl_scale, const float* force_o, const int* inv_order,
                                              int num_movable, int num_filler, const float* pws, const float* area,
                                              const float* lambda_, int num_nodes, const float* v_new, const float* v,
                                              const float* g, float* g_new, double* state, const int* grad_index,
-                                             dp_stream_t stream) {
+                                             cudaStream_t s, int* blocks_out) {
   using namespace dpb;
   DP_REQUIRE(grad_node_order && node_start && wl_scale && force_o && inv_order && pws && area && lambda_ && v_new &&
                  v && g && g_new && state,
              "dp_assemble_precondition_step: null pointer argument");
   DP_REQUIRE(num_nodes > 0 && num_movable >= 0 && num_filler >= 0 && num_movable + num_filler <= num_nodes,
              "dp_assemble_precondition_step: bad node counts");
-  cudaStream_t s = as_stream(stream);
   int blocks = grid_for(num_nodes, kAsmThreads, 4);
   if (blocks > DP_REDUCE_DOUBLES) blocks = DP_REDUCE_DOUBLES;
   double* partials = state + DP_NESTEROV_STATE_DOUBLES;
@@ -481,10 +685,35 @@ extern "C" int dp_assemble_precondition_step(const float* grad_node_order, const
       reinterpret_cast<const float2*>(grad_node_order), node_start, wl_scale, reinterpret_cast<const float2*>(force_o),
       inv_order, num_movable, num_filler, pws, area, lambda_, num_nodes, v_new, v, g, g_new, partials, grad_index,
       trial_gate());
-  int rc = check_launch("dp_assemble_precondition_step");
+  *blocks_out = blocks;
+  return check_launch("dp_assemble_precondition_step");
+}
+
+extern "C" int dp_assemble_precondition_step(const float* grad_node_order, const int* node_start,
+                                             const float* wl_scale, const float* force_o, const int* inv_order,
+                                             int num_movable, int num_filler, const float* pws, const float* area,
+                                             const float* lambda_, int num_nodes, const float* v_new, const float* v,
+                                             const float* g, float* g_new, double* state, const int* grad_index,
+                                             dp_stream_t stream) {
+  using namespace dpb;
+  cudaStream_t s = as_stream(stream);
+  int blocks = 0;
+  int rc = launch_assemble(grad_node_order, node_start, wl_scale, force_o, inv_order, num_movable, num_filler, pws,
+                           area, lambda_, num_nodes, v_new, v, g, g_new, state, grad_index, s, &blocks);
   if (rc) return rc;
-  launch_kernel(nesterov_finish_kernel, 1, 256, 0, s, state, partials, blocks);
+  launch_kernel(nesterov_finish_kernel, 1, 256, 0, s, state, state + DP_NESTEROV_STATE_DOUBLES, blocks);
   return check_launch("dp_assemble_precondition_step finish");
+}
+
+extern "C" int dp_trial_assemble(const float* grad_node_order, const int* node_start, const float* wl_scale,
+                                 const float* force_o, const int* inv_order, int num_movable, int num_filler,
+                                 const float* pws, const float* area, const float* lambda_, int num_nodes,
+                                 const float* v_new, const float* v, const float* g, float* g_new, double* state,
+                                 const int* grad_index, int* norm_blocks, dp_stream_t stream) {
+  DP_REQUIRE(norm_blocks, "dp_trial_assemble: null pointer argument");
+  return launch_assemble(grad_node_order, node_start, wl_scale, force_o, inv_order, num_movable, num_filler, pws, area,
+                         lambda_, num_nodes, v_new, v, g, g_new, state, grad_index, dpb::as_stream(stream),
+                         norm_blocks);
 }
 
 // ============================================================== lane-per-net WA / HPWL
@@ -1008,7 +1237,9 @@ extern "C" int dp_plan_net_lanes(const int* netpin_start_host, int num_nets, con
   return DP_OK;
 }
 
-static int launch_lanes(bool grad, const dpb::LaneArgs& A, double* out_f64, double* hpwl_f64, cudaStream_t s) {
+// blocks_out given: the partials are left for a later finisher, which gets their count
+static int launch_lanes(bool grad, const dpb::LaneArgs& A, double* out_f64, double* hpwl_f64, cudaStream_t s,
+                        int* blocks_out = nullptr) {
   using namespace dpb;
   // one wave: the launch bounds keep 4 blocks of 256 resident per SM, and the
   // warps stride over the groups, so a larger grid only adds a partial last
@@ -1025,6 +1256,10 @@ static int launch_lanes(bool grad, const dpb::LaneArgs& A, double* out_f64, doub
     launch_kernel(wa_lane_kernel<false, false>, blocks, 256, 0, s, A, out_f64 + 1, nullptr, trial_gate());
   int rc = check_launch(grad ? "dp_wa_lanes_forward" : "dp_hpwl_lanes");
   if (rc) return rc;
+  if (blocks_out) {
+    *blocks_out = blocks;
+    return DP_OK;
+  }
   // the WA total and the HPWL (same fixed-order reduction each) in one launch
   if (grad && hpwl_f64) return launch_finish_sum2(out_f64, hpwl_f64, blocks, s);
   return launch_finish_sum(out_f64, blocks, nullptr, s);
@@ -1053,11 +1288,11 @@ static dpb::LaneArgs lane_args(const float* xy, const int* group_deg, const int*
   return A;
 }
 
-extern "C" int dp_wa_lanes_forward(const float* xy, const int* group_deg, const int* group_base, const int* group_net,
+static int wa_lanes(const float* xy, const int* group_deg, const int* group_base, const int* group_net,
                                    int num_groups, const int* ln_node, const float* ln_offx, const float* ln_offy,
                                    const int* ln_csr, const float* net_weights, const unsigned char* net_mask,
                                    const float* inv_gamma, double* wl_f64, float* grad_node_order,
-                                   const unsigned char* hpwl_mask, double* hpwl_f64, dp_stream_t stream) {
+                                   const unsigned char* hpwl_mask, double* hpwl_f64, int* blocks_out, dp_stream_t stream) {
   DP_REQUIRE(xy && group_deg && group_base && group_net && ln_node && ln_offx && ln_offy && net_mask && inv_gamma &&
                  wl_f64 && grad_node_order,
              "dp_wa_lanes_forward: null pointer argument");
@@ -1067,7 +1302,27 @@ extern "C" int dp_wa_lanes_forward(const float* xy, const int* group_deg, const 
   DP_REQUIRE(num_groups >= 0, "dp_wa_lanes_forward: bad group count");
   const dpb::LaneArgs A = lane_args(xy, group_deg, group_base, group_net, num_groups, ln_node, ln_offx, ln_offy,
                                     ln_csr, net_weights, net_mask, hpwl_mask, inv_gamma, grad_node_order);
-  return launch_lanes(true, A, wl_f64, hpwl_f64, dpb::as_stream(stream));
+  return launch_lanes(true, A, wl_f64, hpwl_f64, dpb::as_stream(stream), blocks_out);
+}
+
+extern "C" int dp_wa_lanes_forward(const float* xy, const int* group_deg, const int* group_base, const int* group_net,
+                                   int num_groups, const int* ln_node, const float* ln_offx, const float* ln_offy,
+                                   const int* ln_csr, const float* net_weights, const unsigned char* net_mask,
+                                   const float* inv_gamma, double* wl_f64, float* grad_node_order,
+                                   const unsigned char* hpwl_mask, double* hpwl_f64, dp_stream_t stream) {
+  return wa_lanes(xy, group_deg, group_base, group_net, num_groups, ln_node, ln_offx, ln_offy, ln_csr, net_weights,
+                  net_mask, inv_gamma, wl_f64, grad_node_order, hpwl_mask, hpwl_f64, nullptr, stream);
+}
+
+extern "C" int dp_trial_wirelength(const float* xy, const int* group_deg, const int* group_base, const int* group_net,
+                                   int num_groups, const int* ln_node, const float* ln_offx, const float* ln_offy,
+                                   const int* ln_csr, const float* net_weights, const unsigned char* net_mask,
+                                   const float* inv_gamma, double* wl_f64, float* grad_node_order,
+                                   const unsigned char* hpwl_mask, double* hpwl_f64, int* wa_blocks,
+                                   dp_stream_t stream) {
+  DP_REQUIRE(hpwl_f64 && wa_blocks, "dp_trial_wirelength: null pointer argument");
+  return wa_lanes(xy, group_deg, group_base, group_net, num_groups, ln_node, ln_offx, ln_offy, ln_csr, net_weights,
+                  net_mask, inv_gamma, wl_f64, grad_node_order, hpwl_mask, hpwl_f64, wa_blocks, stream);
 }
 
 extern "C" int dp_hpwl_lanes(const float* xy, const int* group_deg, const int* group_base, const int* group_net,

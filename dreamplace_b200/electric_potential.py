@@ -106,11 +106,12 @@ class PoissonWorkspace(object):
         return self
 
 
-def _poisson_spectral(rho, bin_size_x, bin_size_y, prec, energy, rho_scale=1.0, ws=None):
+def _poisson_spectral(rho, bin_size_x, bin_size_y, prec, energy, rho_scale=1.0, ws=None, prepared=False):
     """G1 and G2 of the solve: the two spectral operands a*wx, a*wy [M, N];
     when ``energy`` (f64[1]) is given the G2 epilogue adds the energy to it.
     The solve runs on rho * rho_scale (the scale is G1's alpha).  With a
-    PoissonWorkspace ``ws`` the operands are the workspace's."""
+    PoissonWorkspace ``ws`` the operands are the workspace's (``prepared``: the
+    map's operand is filled already)."""
     M, N = rho.shape
     dev = rho.device
     cM = transform_matrices(M, prec, dev)[0]
@@ -121,7 +122,7 @@ def _poisson_spectral(rho, bin_size_x, bin_size_y, prec, energy, rho_scale=1.0, 
     if prec == 0:
         g1["a_hi"] = rho
     elif ws is not None:
-        ws.rho.fill(rho).as_a(g1)
+        (ws.rho if prepared else ws.rho.fill(rho)).as_a(g1)
     else:
         Operand.from_tensor(rho, prec).as_a(g1)
     cN.as_b(g1)
@@ -168,7 +169,8 @@ def _poisson_fft(rho, bin_size_x, bin_size_y, rho_scale, work, ex, ey, energy, w
                   fft_table(rho.size(1), dev), work, ex, ey, energy, bool(want_energy))
 
 
-def poisson_solve(rho, bin_size_x, bin_size_y, precision, fast_mode=False, rho_scale=1.0, ws=None, fast=True):
+def poisson_solve(rho, bin_size_x, bin_size_y, precision, fast_mode=False, rho_scale=1.0, ws=None, fast=True,
+                  prepared=False):
     """Field maps and energy of a normalised density map ``rho`` [M, N] (fp32).
 
     Returns (field_map_x, field_map_y, energy_f64[1]); energy is zero when
@@ -177,7 +179,8 @@ def poisson_solve(rho, bin_size_x, bin_size_y, precision, fast_mode=False, rho_s
     density map and rho_scale = 1 / bin area give the solve of rho.  With a
     PoissonWorkspace ``ws`` nothing is allocated and the results are the
     workspace's buffers.  fast False: the matrix products, also where the fast
-    transforms would serve the map."""
+    transforms would serve the map.  prepared: the caller filled ws.rho (where
+    the products read it) and zeroed ws.energy."""
     prec = precision_code(precision)
     M, N = rho.shape
     dev = rho.device
@@ -198,10 +201,12 @@ def poisson_solve(rho, bin_size_x, bin_size_y, precision, fast_mode=False, rho_s
     if ws is not None:
         ws.products()
         energy = ws.energy
-        C.zero_(energy)
+        if not prepared:
+            C.zero_(energy)
     else:
         energy = torch.zeros(1, dtype=torch.float64, device=dev)
-    spec = _poisson_spectral(rho, bin_size_x, bin_size_y, prec, None if fast_mode else energy, rho_scale, ws)
+    spec = _poisson_spectral(rho, bin_size_x, bin_size_y, prec, None if fast_mode else energy, rho_scale, ws,
+                             prepared)
     # G3: U^T = (A R^T)^T for the x field (R = Ch_N) and the y field (Sh_N)
     rights = [chN, shN]
     us = ws.us if ws is not None else [Operand((N, M), prec, dev) for _ in spec]

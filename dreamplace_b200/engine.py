@@ -131,6 +131,7 @@ class GPEngine(object):
         self.O = [torch.zeros(REDUCE_DOUBLES, **f64) for _ in range(NSLOT)]
         self.metrics = [torch.zeros(8, **f64) for _ in range(NSLOT)]
         self.metrics_host = [torch.zeros(8, dtype=torch.float64, pin_memory=True) for _ in range(NSLOT)]
+        self.metrics_dev = [C.host_pointer(t) for t in self.metrics_host]
         self.ready = [None] * NSLOT
         self.grad_scale = torch.zeros(1, dtype=torch.float32, device=dev)
         # (density factor, quadratic penalty coefficient) read by the objective
@@ -143,7 +144,11 @@ class GPEngine(object):
         self.ovf_area = float(self.ovf_op.bin_size_x * self.ovf_op.bin_size_y)
         self.ovf_target = float(self.ovf_op.target_density) * self.ovf_area
         self.det = bool(params.deterministic_flag)
-        self.scratch = torch.empty(ep.num_bins_x * ep.num_bins_y, dtype=torch.int64, device=dev) if self.det else None
+        # deterministic mode: the int64 sums of the movable cells and of the
+        # fillers (a scatter outside a trial uses the first)
+        bins = ep.num_bins_x * ep.num_bins_y
+        self.scratch2 = torch.empty(2 * bins, dtype=torch.int64, device=dev) if self.det else None
+        self.scratch = self.scratch2[:bins] if self.det else None
         self.prec = precision_code(ep.precision)
         # the Poisson solve's operands and outputs, allocated once: every trial
         # (eager or captured) of this design solves on its one stream.  split_bf16
@@ -399,30 +404,55 @@ class GPEngine(object):
         field force is gathered in visiting order and assembled per node together
         with the wirelength pin sum, the preconditioner and the norms (one pass
         over the nodes).  The HPWL and overflow of v_new land in the metric
-        buffers of slot s + 1."""
-        ep = self.ep
+        buffers of slot s + 1.  dp_trial_start has zeroed the density sums and
+        the energy; dp_trial_finish ends every sum and fills the metrics row,
+        also the host's."""
+        ep, dc, d = self.ep, self.data, self.design
         q_new = (s + 1) % NSLOT
         w = self.weights[s]
         # (the WA forward was also run on a second stream beside the density
         # chain: its kernels and the scatter's, or the GEMMs', slow each other
         # down by about what they would overlap, ~1% net, so it runs in line)
         self._mark("wa_forward", 0)
-        self.wirelength(v_new, self.H[q_new], w[2:3])
+        wa_blocks = C.trial_wirelength(self.xy(v_new), self.group_deg, self.group_base, self.group_net, self.ln_node,
+                                       self.ln_offx, self.ln_offy,
+                                       self.ln_csr if self.lane_of_csr is None else None, dc.net_weights,
+                                       dc.net_mask_ignore_large_degrees, w[2:3], self.wl64_buf, self.gnode,
+                                       dc.net_mask_all, self.H[q_new])
         self._mark("wa_forward", 1)
         self._mark("density_scatter", 0)
-        self.scatter_maps(v_new, self.O[q_new])
+        xy_o, order = self._cells_xy(v_new)
+        # the solve's first product reads the map as a hi + lo bf16 operand, which
+        # the pass that finishes the map then writes too
+        op = self.poisson_ws.rho if self.prec == 3 and self.poisson_ws.fft_work is None else None
+        ovf_blocks = C.trial_density(xy_o, order, self.rec4, self.ratio_o, ep.num_movable_nodes, self.order.numel(),
+                                     ep.initial_density_map.view(-1), float(ep.xl), float(ep.yl), float(ep.xh),
+                                     float(ep.yh), float(ep.bin_size_x), float(ep.bin_size_y), ep.num_bins_x,
+                                     ep.num_bins_y, int(self.det), self.scratch2, self.omap.view(-1),
+                                     self.dmap.view(-1), op.hi if op is not None else None,
+                                     op.lo if op is not None else None, self.ovf_target, self.O[q_new])
         self._mark("density_scatter", 1)
         self._mark("poisson_gemms", 0)
+        if op is None and self.poisson_ws.fft_work is None and self.prec != 0:
+            self.poisson_ws.rho.fill(self.dmap)
         # rho = D / bin area is applied as the first GEMM's alpha
         ex, ey, energy = poisson_solve(self.dmap, ep.bin_size_x, ep.bin_size_y, self.prec, bool(ep.fast_mode),
-                                       1.0 / (ep.bin_size_x * ep.bin_size_y), self.poisson_ws)
+                                       1.0 / (ep.bin_size_x * ep.bin_size_y), self.poisson_ws, prepared=True)
         self._mark("poisson_gemms", 1)
-        C.objective_finish(self.wl64, energy, w[0:1], self.factor_quad, self.obj64, self.grad_scale)
         self._mark("field_gather", 0)
-        self.field_force(v_new, ex, ey)
+        C.trial_force(energy, w[0:1], self.factor_quad, ex.view(-1), ey.view(-1), xy_o, order, self.rec4,
+                      self.ratio_o, self.order.numel(), float(ep.xl), float(ep.yl), float(ep.bin_size_x),
+                      float(ep.bin_size_y), ep.num_bins_x, ep.num_bins_y, -1.0, self.force_o)
         self._mark("field_gather", 1)
         self._mark("assemble_precondition", 0)
-        self.assemble(v, g, v_new, g_new, s)
+        norm_blocks = C.trial_assemble(self.gnode, self.node_start, self.one, self.force_o, self.inv_order,
+                                       d.num_movable_nodes, d.num_filler_nodes, self._pws(), dc.node_areas, w[0:1],
+                                       v_new, v, g, g_new, self.S[s], self.lane_of_csr)
+        # the metrics row: HPWL / overflow of v_k (computed when v_k was the trial
+        # point) and the trial's scalars, on the device and in the host's pinned copy
+        C.trial_finish(self.wl64_buf, self.H[q_new], wa_blocks, self.O[q_new], ovf_blocks, self.ovf_area, energy,
+                       w[0:1], self.factor_quad, self.S[s], norm_blocks, self.H[s], self.O[s], self.obj64,
+                       self.metrics[s], self.metrics_dev[s])
         self._mark("assemble_precondition", 1)
         self.last_energy = energy
         return energy
@@ -562,22 +592,22 @@ class GPEngine(object):
         the device (advance, density weight, gamma from slot s - 1)."""
         t = (s + 1) % NSLOT
         self._mark_slot = s
-        gate = self.gate if self.use_graphs else None
-        if head:
-            r = (s - 1) % NSLOT
-            C.iteration_head(self.S[r], self.S[s], self.sched[r], self.sched[s], self.H[r][0:1], self.O[r][0:1],
-                             self.weights[r], self.weights[s], *self.head_scalars, gate=gate)
-        elif gate is not None:
-            C.trial_gate(gate)
-        v, g = self.V[s], self.G[s]
-        vn, gn = self.V[t], self.G[t]
-        st = self.S[s]
+        r = (s - 1) % NSLOT
+        d = self.design
+        scatter_write = self.xyo_mode == "trial"
+        zero = [self.scratch2] if self.det else [self.omap, self.dmap]
         self._mark("nesterov_trial", 0)
-        self.nesterov_trial_only(s)
+        C.trial_start([self.S[r], self.sched[r], self.sched[s], self.H[r][0:1], self.O[r][0:1], self.weights[r],
+                       self.weights[s]] if head else None, self.head_scalars,
+                      self.gate if self.use_graphs else None, self.V[s], self.G[s], self.U[s], self.U[t], self.V[t],
+                      self.XY[t], self.S[s], self.data.node_size_x, self.data.node_size_y, float(d.xl), float(d.yl),
+                      float(d.xh), float(d.yh), d.num_movable_nodes, d.num_filler_nodes,
+                      self.inv_order if scatter_write else None, self.XYO[t] if scatter_write else None, zero,
+                      self.poisson_ws.energy, self.O[t][2:3])
+        if self.xyo_mode == "gather":
+            C.gather_order_xy(self.XY[t], self.order, self.order.numel(), self.XYO[t])
         self._mark("nesterov_trial", 1)
-        energy = self.objective_and_step(v, g, vn, gn, s)
-        # HPWL / overflow of v_k (computed when v_k was the trial point), then the trial's scalars
-        C.trial_metrics(self.H[s], self.O[s], st, self.obj64, self.wl64, energy, self.metrics[s])
+        self.objective_and_step(self.V[s], self.G[s], self.V[t], self.G[t], s)
 
     def nesterov_trial_only(self, s):
         """The trial point from slot s into slot s + 1, and its visiting-order
@@ -599,8 +629,6 @@ class GPEngine(object):
         # reference's per-iteration move_boundary(pos) is the identity here,
         # and its evaluation (HPWL, overflow) was computed with it
         self._trial(s, head)
-        # the metrics' read-back is part of the trial (a copy node in the graph)
-        self.metrics_host[s].copy_(self.metrics[s], non_blocking=True)
 
     def _graph(self, s, head, warm=True):
         key = (s, head)

@@ -508,6 +508,61 @@ int dp_scatter_pairs_to_nodes(const float* vals_o, const int* order, int count, 
  * counterpart). */
 int dp_trial_metrics(const double* hpwl, const double* overflow2, const double* state, const double* obj,
                      const double* wl, const double* energy, double* out8, dp_stream_t stream);
+/* ---- one Nesterov trial in as few launches as it needs ------------------------
+ * The kernels of dp_iteration_head, dp_nesterov_trial, dp_wa_lanes_forward,
+ * dp_density_map_ordered_split, dp_prepare_operand, dp_electric_force_ordered,
+ * dp_assemble_precondition_step, dp_objective_finish and dp_trial_metrics with
+ * their one-block finishers, memsets and scalar kernels folded together; the
+ * same values.  Order: dp_trial_start, dp_trial_wirelength, dp_trial_density,
+ * the solve (energy summed onto the zeroed word), dp_trial_force,
+ * dp_trial_assemble, dp_trial_finish.
+ *
+ * dp_trial_start: the iteration head (state_prev .. upper; skipped with
+ * state_prev NULL, whose gate word is then set to 0) and the trial point, and
+ * zeroes two ranges (16-byte aligned, whole words) and two doubles. */
+int dp_trial_start(const double* state_prev, const double* sched_prev, double* sched_new, const double* hpwl_k,
+                   const double* overflow_k, const float* weights_prev, float* weights_new, double base_gamma,
+                   double total_area, double ref_hpwl, double lower, double upper, int* gate, const float* v,
+                   const float* g, const float* u, float* u_new, float* v_new, float* xy_new, double* state,
+                   const float* node_size_x, const float* node_size_y, float xl, float yl, float xh, float yh,
+                   int num_nodes, int num_movable, int num_filler, const int* inv_order, float* xy_order, void* zero0,
+                   size_t zero0_bytes, void* zero1, size_t zero1_bytes, double* zero_cell0, double* zero_cell1,
+                   dp_stream_t stream);
+/* dp_wa_lanes_forward with the partials left in wl_f64 / hpwl_f64 (*wa_blocks of them) */
+int dp_trial_wirelength(const float* xy, const int* group_deg, const int* group_base, const int* group_net,
+                        int num_groups, const int* ln_node, const float* ln_offx, const float* ln_offy,
+                        const int* ln_csr, const float* net_weights, const unsigned char* net_mask,
+                        const float* inv_gamma, double* wl_f64, float* grad_node_order,
+                        const unsigned char* hpwl_mask, double* hpwl_f64, int* wa_blocks, dp_stream_t stream);
+/* dp_density_map_ordered_split onto zeroed sums (out_first and out_all, or in
+ * deterministic mode scratch2: two int64 maps) with overflow[2] zeroed; all_hi /
+ * all_lo (optional): out_all as a split-BF16 operand; *overflow_blocks partials
+ * are left from overflow[3]. */
+int dp_trial_density(const float* xy_o, const int* order, const float* rec4, const float* ratio_o, int num_first,
+                     int count, const float* initial_density_map, float xl, float yl, float xh, float yh,
+                     float bin_size_x, float bin_size_y, float inv_bin_size_x, float inv_bin_size_y, int num_bins_x,
+                     int num_bins_y, int deterministic, int fraction_bits, int64_t* scratch2, float* out_first,
+                     float* out_all, void* all_hi, void* all_lo, double target_area, double* overflow,
+                     int* overflow_blocks, dp_stream_t stream);
+/* dp_electric_force_ordered with the scale formed from the energy as dp_objective_finish does */
+int dp_trial_force(const double* energy, const float* density_weight, const float* factor_quad, int num_bins_x,
+                   int num_bins_y, const float* field_map_x, const float* field_map_y, const float* xy_o,
+                   const int* order, const float* rec4, const float* ratio_o, int count, float xl, float yl,
+                   float bin_size_x, float bin_size_y, float inv_bin_size_x, float inv_bin_size_y, float scale,
+                   float* force_o, dp_stream_t stream);
+/* dp_assemble_precondition_step with the norms left as *norm_blocks partials in state */
+int dp_trial_assemble(const float* grad_node_order, const int* node_start, const float* wl_scale,
+                      const float* force_o, const int* inv_order, int num_movable, int num_filler, const float* pws,
+                      const float* area, const float* lambda_, int num_nodes, const float* v_new, const float* v,
+                      const float* g, float* g_new, double* state, const int* grad_index, int* norm_blocks,
+                      dp_stream_t stream);
+/* every sum of the trial, the objective, the step-size test and the metrics row
+ * of dp_trial_metrics (hpwl_v, overflow_v: those of v_k); out8_host (optional):
+ * a device pointer to pinned host memory that receives the row too. */
+int dp_trial_finish(double* wl, double* hpwl, int wa_blocks, double* overflow, int overflow_blocks, double bin_area,
+                    const double* energy, const float* density_weight, const float* factor_quad, double* state,
+                    int norm_blocks, const double* hpwl_v, const double* overflow_v, double* obj, double* out8,
+                    double* out8_host, dp_stream_t stream);
 /* Zeroes bytes at ptr on the stream (a memset, no kernel). */
 int dp_zero(void* ptr, size_t bytes, dp_stream_t stream);
 

@@ -256,3 +256,49 @@ def test_profile_piece_runs_every_piece():
     from dreamplace_b200 import profile_piece
     for piece in profile_piece.PIECES:
         profile_piece.main(["--piece", piece, "--design", "cells_10k", "--iterations", "3", "--repeat", "1"])
+
+
+@pytest.mark.parametrize("precision,deterministic", [("split_bf16", 1), ("split_bf16", 0), ("fp32", 1), ("tf32", 1)])
+def test_fused_trial_equals_its_pieces(design, precision, deterministic):
+    """A trial through dp_trial_* (head, zeroing, finishers and scalar kernels
+    folded into the heavy kernels) against the stand-alone entry points launched
+    one by one: every sum keeps its order, so deterministic maps give the same
+    bits; fp32 atomics may add in another order (1e-4 of the largest entry)."""
+    from dreamplace_b200._native import C
+    from dreamplace_b200.electric_potential import poisson_solve
+    placer, _, _ = run(design, "graph", precision, 6, deterministic=deterministic)
+    eng = placer.stepper.eng
+    ep, d = eng.ep, eng.design
+    torch.cuda.synchronize()
+    s = eng.slot
+    r, t = (s - 1) % 3, (s + 1) % 3
+    # an iteration ahead may have run from slot s: start from its inputs
+    eng._trial(s, head=True)
+    torch.cuda.synchronize()
+    names = ("V", "U", "G", "XY", "XYO")
+    got = {k: getattr(eng, k)[t].clone() for k in names}
+    got.update(row=eng.metrics[s].clone(), host=eng.metrics_host[s].clone().cuda(), state=eng.S[s][:8].clone(),
+               weights=eng.weights[s].clone(), sched=eng.sched[s].clone(), hpwl=eng.H[t][0].clone(),
+               ovf=eng.O[t][:2].clone())
+    for k in names:
+        getattr(eng, k)[t].fill_(-1.0)
+    C.iteration_head(eng.S[r], eng.S[s], eng.sched[r], eng.sched[s], eng.H[r][0:1], eng.O[r][0:1], eng.weights[r],
+                     eng.weights[s], *eng.head_scalars, gate=eng.gate)
+    assert eng.gate.item() == 0
+    eng.nesterov_trial_only(s)
+    w = eng.weights[s]
+    eng.wirelength(eng.V[t], eng.H[t], w[2:3])
+    eng.scatter_maps(eng.V[t], eng.O[t])
+    ex, ey, energy = poisson_solve(eng.dmap, ep.bin_size_x, ep.bin_size_y, eng.prec, bool(ep.fast_mode),
+                                   1.0 / (ep.bin_size_x * ep.bin_size_y), eng.poisson_ws)
+    C.objective_finish(eng.wl64, energy, w[0:1], eng.factor_quad, eng.obj64, eng.grad_scale)
+    eng.field_force(eng.V[t], ex, ey)
+    eng.assemble(eng.V[s], eng.G[s], eng.V[t], eng.G[t], s)
+    C.trial_metrics(eng.H[s], eng.O[s], eng.S[s], eng.obj64, eng.wl64, energy, eng.metrics[s])
+    want = {k: getattr(eng, k)[t] for k in names}
+    want.update(row=eng.metrics[s], host=eng.metrics[s], state=eng.S[s][:8], weights=eng.weights[s],
+                sched=eng.sched[s], hpwl=eng.H[t][0], ovf=eng.O[t][:2])
+    for k, v in want.items():
+        # the energy is an atomic fp64 sum of the solve's tiles: its last bits vary
+        rel = 1e-12 if deterministic and k in ("row", "host") else 0.0 if deterministic else 1e-4
+        assert (got[k].double() - v.double()).abs().max() <= rel * v.double().abs().max(), k
