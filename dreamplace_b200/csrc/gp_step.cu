@@ -1364,15 +1364,26 @@ __global__ void wa_pins_backward_kernel(const float2* __restrict__ grad_lane, co
                                         int num_pins, float* __restrict__ gx, float* __restrict__ gy) {
   grid_dep_sync();
   const float g = grad_out[0];
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < num_pins; p += gridDim.x * blockDim.x) {
-    float x = 0.f, y = 0.f;
-    if (!(pin_mask && pin_mask[p])) {
-      const float2 v = __ldg(grad_lane + __ldg(lane_of_pin + p));
-      x = fmul(v.x, g);
-      y = fmul(v.y, g);
+  // four pins of a thread in flight (pin -> lane slot -> gradient)
+  const int stride = gridDim.x * blockDim.x;
+  for (int p0 = blockIdx.x * blockDim.x + threadIdx.x; p0 < num_pins; p0 += 4 * stride) {
+    int at[4];
+    float2 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long p = p0 + (long long)u * stride;
+      at[u] = p < num_pins && !(pin_mask && pin_mask[p]) ? __ldcs(lane_of_pin + p) : -1;
     }
-    __stcs(gx + p, x);
-    __stcs(gy + p, y);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = at[u] >= 0 ? __ldg(grad_lane + at[u]) : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long p = p0 + (long long)u * stride;
+      if (p < num_pins) {
+        gx[p] = at[u] >= 0 ? fmul(v[u].x, g) : 0.f;
+        gy[p] = at[u] >= 0 ? fmul(v[u].y, g) : 0.f;
+      }
+    }
   }
 }
 }  // namespace dpb

@@ -123,59 +123,130 @@ __global__ void wa_merged_backward_kernel(const float* __restrict__ grad_pos,
   }
 }
 
-__global__ void pin_pos_forward_kernel(const float* __restrict__ x, const float* __restrict__ y,
-                                       const float* __restrict__ offx, const float* __restrict__ offy,
-                                       const int* __restrict__ pin2node, int num_pins,
-                                       float* __restrict__ pin_x, float* __restrict__ pin_y) {
+// Four pins of a thread in flight: pin -> node -> position is a chain of two
+// dependent reads, so the time is theirs, not the bytes'.  MEASURED_PPF
+__global__ void __launch_bounds__(256) pin_pos_forward_kernel(
+    const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ offx,
+    const float* __restrict__ offy, const int* __restrict__ pin2node, int num_pins, float* __restrict__ pin_x,
+    float* __restrict__ pin_y) {
   grid_dep_sync();
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < num_pins; p += gridDim.x * blockDim.x) {
-    int n = pin2node[p];
+  const int stride = gridDim.x * blockDim.x;
+  int p = blockIdx.x * blockDim.x + threadIdx.x;
+  for (; (long long)p + 3ll * stride < num_pins; p += 4 * stride) {
+    int n[4];
+    float vx[4], vy[4], ox[4], oy[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) n[u] = __ldcs(pin2node + p + u * stride);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      vx[u] = x[n[u]];
+      vy[u] = y[n[u]];
+      ox[u] = __ldcs(offx + p + u * stride);
+      oy[u] = __ldcs(offy + p + u * stride);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      pin_x[p + u * stride] = fadd(ox[u], vx[u]);
+      pin_y[p + u * stride] = fadd(oy[u], vy[u]);
+    }
+  }
+  for (; p < num_pins; p += stride) {
+    const int n = pin2node[p];
     pin_x[p] = fadd(offx[p], x[n]);
     pin_y[p] = fadd(offy[p], y[n]);
   }
 }
 
-__global__ void pin_pos_backward_kernel(const float* __restrict__ gpx, const float* __restrict__ gpy,
-                                        const int* __restrict__ flat_node2pin,
-                                        const int* __restrict__ node_start, int num_physical,
-                                        int num_nodes, float* __restrict__ gx, float* __restrict__ gy) {
-  grid_dep_sync();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < num_nodes; i += gridDim.x * blockDim.x) {
-    float sx = 0.f, sy = 0.f;
-    if (i < num_physical) {
-      int b = node_start[i], e = node_start[i + 1];
-      for (int j = b; j < e; ++j) {
-        int p = flat_node2pin[j];
-        sx = fadd(sx, gpx[p]);
-        sy = fadd(sy, gpy[p]);
-      }
+// One warp per tile of 32 consecutive segments (a node's pins, a net's pins)
+// of a CSR: the tile's entries [p0, p1) are one contiguous range, gathered
+// kFoldPins at a time into the warp's buffer with four independent gathers a
+// lane, and each lane folds its own segment's entries [my0, my1) in order.  A
+// thread walking its own segment instead has one dependent gather in flight,
+// at an address no neighbour shares.
+constexpr int kFoldThreads = 256;
+constexpr int kFoldPins = 128;
+
+template <typename Fold>
+__device__ __forceinline__ void warp_fold(float2* stage, const int* __restrict__ flat, const float* __restrict__ px,
+                                          const float* __restrict__ py, int lane, int p0, int p1, int my0, int my1,
+                                          Fold fold) {
+  for (int c0 = p0; c0 < p1; c0 += kFoldPins) {
+    int id[kFoldPins / 32];
+    float2 q[kFoldPins / 32];
+#pragma unroll
+    for (int j = 0; j < kFoldPins / 32; ++j) {
+      const int k = c0 + 32 * j + lane;
+      id[j] = k < p1 ? __ldcs(flat + k) : -1;
     }
-    gx[i] = sx;
-    gy[i] = sy;
+#pragma unroll
+    for (int j = 0; j < kFoldPins / 32; ++j)
+      q[j] = id[j] >= 0 ? make_float2(__ldg(px + id[j]), __ldg(py + id[j])) : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < kFoldPins / 32; ++j) stage[32 * j + lane] = q[j];
+    __syncwarp();
+    const int ka = max(my0, c0), kb = min(my1, c0 + kFoldPins);
+    for (int k = ka; k < kb; ++k) fold(stage[k - c0]);
+    __syncwarp();  // refilled by the next chunk or tile
   }
 }
 
-__global__ void __launch_bounds__(256) hpwl_kernel(const float* __restrict__ px, const float* __restrict__ py,
-                                                   const int* __restrict__ flat_netpin,
-                                                   const int* __restrict__ netpin_start, int num_nets,
-                                                   const float* __restrict__ net_weights,
-                                                   const unsigned char* __restrict__ net_mask,
-                                                   double* __restrict__ partials) {
+// MEASURED_PPB
+__global__ void __launch_bounds__(kFoldThreads) pin_pos_backward_kernel(
+    const float* __restrict__ gpx, const float* __restrict__ gpy, const int* __restrict__ flat_node2pin,
+    const int* __restrict__ node_start, int num_physical, int num_nodes, float* __restrict__ gx,
+    float* __restrict__ gy) {
   grid_dep_sync();
+  __shared__ float2 stage[kFoldThreads / 32][kFoldPins];
+  const int lane = threadIdx.x & 31;
+  const int warp = (blockIdx.x * kFoldThreads + threadIdx.x) >> 5, nwarps = (gridDim.x * kFoldThreads) >> 5;
+  for (int n0 = warp * 32; n0 < num_nodes; n0 += nwarps * 32) {
+    const int i = n0 + lane;
+    float sx = 0.f, sy = 0.f;
+    const int cnt = min(num_physical - n0, 32);  // nodes of the tile with pins (warp-uniform)
+    if (cnt > 0) {
+      const int my0 = i < num_physical ? node_start[i] : 0, my1 = i < num_physical ? node_start[i + 1] : 0;
+      const int p0 = __shfl_sync(0xffffffffu, my0, 0), p1 = __shfl_sync(0xffffffffu, my1, cnt - 1);
+      warp_fold(stage[threadIdx.x >> 5], flat_node2pin, gpx, gpy, lane, p0, p1, my0, my1, [&](float2 v) {
+        sx = fadd(sx, v.x);
+        sy = fadd(sy, v.y);
+      });
+    }
+    if (i < num_nodes) {
+      gx[i] = sx;
+      gy[i] = sy;
+    }
+  }
+}
+
+// MEASURED_HPWL
+__global__ void __launch_bounds__(kFoldThreads) hpwl_kernel(const float* __restrict__ px, const float* __restrict__ py,
+                                                            const int* __restrict__ flat_netpin,
+                                                            const int* __restrict__ netpin_start, int num_nets,
+                                                            const float* __restrict__ net_weights,
+                                                            const unsigned char* __restrict__ net_mask,
+                                                            double* __restrict__ partials) {
+  grid_dep_sync();
+  __shared__ float2 stage[kFoldThreads / 32][kFoldPins];
+  const int lane = threadIdx.x & 31;
+  const int warp = (blockIdx.x * kFoldThreads + threadIdx.x) >> 5, nwarps = (gridDim.x * kFoldThreads) >> 5;
   double c = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < num_nets; i += gridDim.x * blockDim.x) {
-    if (net_mask[i]) {
-      float max_x = -FLT_MAX, min_x = FLT_MAX, max_y = -FLT_MAX, min_y = FLT_MAX;
-      for (int j = netpin_start[i]; j < netpin_start[i + 1]; ++j) {
-        int p = flat_netpin[j];
-        float xx = px[p], yy = py[p];
-        min_x = fminf(min_x, xx);
-        max_x = fmaxf(max_x, xx);
-        min_y = fminf(min_y, yy);
-        max_y = fmaxf(max_y, yy);
-      }
+  for (int n0 = warp * 32; n0 < num_nets; n0 += nwarps * 32) {
+    const int i = n0 + lane, cnt = min(num_nets - n0, 32);
+    const bool live = i < num_nets;
+    const int my0 = live ? netpin_start[i] : 0, my1 = live ? netpin_start[i + 1] : 0;
+    const bool on = live && net_mask[i];
+    const float w = on && net_weights ? net_weights[i] : 1.f;
+    const int p0 = __shfl_sync(0xffffffffu, my0, 0), p1 = __shfl_sync(0xffffffffu, my1, cnt - 1);
+    float max_x = -FLT_MAX, min_x = FLT_MAX, max_y = -FLT_MAX, min_y = FLT_MAX;
+    warp_fold(stage[threadIdx.x >> 5], flat_netpin, px, py, lane, p0, p1, my0, my1, [&](float2 v) {
+      min_x = fminf(min_x, v.x);
+      max_x = fmaxf(max_x, v.x);
+      min_y = fminf(min_y, v.y);
+      max_y = fmaxf(max_y, v.y);
+    });
+    if (on) {
       float h = fsub(fadd(fsub(max_x, min_x), max_y), min_y);
-      if (net_weights) h = fmul(h, net_weights[i]);
+      if (net_weights) h = fmul(h, w);
       c += (double)h;
     }
   }
@@ -264,7 +335,7 @@ extern "C" int dp_pin_pos_backward(const float* grad_pin, int num_pins, const in
   DP_REQUIRE(grad_pin && flat_node2pin && node_start && grad_pos, "dp_pin_pos_backward: null pointer argument");
   DP_REQUIRE(num_physical <= num_nodes, "dp_pin_pos_backward: num_physical_nodes > num_nodes");
   if (num_nodes == 0) return DP_OK;
-  launch_kernel(pin_pos_backward_kernel, grid_for(num_nodes, 256, 8), 256, 0, as_stream(stream), 
+  launch_kernel(pin_pos_backward_kernel, grid_for(num_nodes, kFoldThreads, 8), kFoldThreads, 0, as_stream(stream), 
       grad_pin, grad_pin + num_pins, flat_node2pin, node_start, num_physical, num_nodes, grad_pos,
       grad_pos + num_nodes);
   return check_launch("dp_pin_pos_backward");
