@@ -316,25 +316,25 @@ __global__ void __launch_bounds__(kReduceThreads) trial_finish_kernel(TrialFinis
   const double* src[5] = {a.wl + 1, a.hpwl + 1, a.ovf + 3, a.st + DP_NESTEROV_STATE_DOUBLES,
                           a.st + DP_NESTEROV_STATE_DOUBLES + a.norm_blocks};
   const int cnt[5] = {a.wa_blocks, a.wa_blocks, a.ovf_blocks, a.norm_blocks, a.norm_blocks};
-  double v[5];
+  // every load of the five sums is in flight before the first add
+  double x[5][kStridedLoads];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) strided_load(x[k], src[k], cnt[k]);
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
-    v[k] = 0.0;
-    for (int i = threadIdx.x; i < cnt[k]; i += kReduceThreads) v[k] += src[k][i];
-  }
-#pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    v[k] = warp_sum(v[k]);
-    if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = v[k];
+    const double v = warp_sum(strided_sum(x[k]));
+    if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = v;
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
+  if (threadIdx.x >= 32) return;
+  // lane k adds the warp totals of sum k in warp order
+  double mine = 0.0;
+  if (threadIdx.x < 5)
+    for (int w = 0; w < kReduceThreads / 32; ++w) mine += sh[threadIdx.x][w];
   double r[5];
 #pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    r[k] = 0.0;
-    for (int w = 0; w < kReduceThreads / 32; ++w) r[k] += sh[k][w];
-  }
+  for (int k = 0; k < 5; ++k) r[k] = __shfl_sync(0xffffffffu, mine, k);
+  if (threadIdx.x != 0) return;
   a.wl[0] = r[0];
   a.hpwl[0] = r[1];
   a.ovf[0] = r[2];

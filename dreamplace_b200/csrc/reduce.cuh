@@ -30,14 +30,35 @@ __device__ __forceinline__ void block_partial(double a, double* partials) {
   __syncthreads();
 }
 
+// the thread's strided partial sum of partials[0 .. count).  The loads of the
+// first kStridedLoads strides go out together: one after another, each waiting
+// for the last one's add, three rounds of L2 misses were most of a one-block
+// finisher's time
+constexpr int kStridedLoads = 5;  // DP_REDUCE_DOUBLES / kReduceThreads: all there can be
+
+__device__ __forceinline__ void strided_load(double (&x)[kStridedLoads], const double* partials, int count) {
+#pragma unroll
+  for (int u = 0; u < kStridedLoads; ++u) {
+    const int i = threadIdx.x + u * kReduceThreads;
+    x[u] = i < count ? partials[i] : 0.0;
+  }
+}
+
+__device__ __forceinline__ double strided_sum(const double (&x)[kStridedLoads]) {
+  double v = 0.0;
+#pragma unroll
+  for (int u = 0; u < kStridedLoads; ++u) v += x[u];
+  return v;
+}
+
 // every thread returns the same total: strided per-thread sums, an xor
 // butterfly per warp (identical in every lane), then the warp totals in warp
-// order; a fixed order, two block barriers
+// order; a fixed order, two block barriers.  count <= DP_REDUCE_DOUBLES
 __device__ __forceinline__ double finish_sum(const double* partials, int count) {
   __shared__ double sh[kReduceThreads / 32];
-  double v = 0.0;
-  for (int i = threadIdx.x; i < count; i += kReduceThreads) v += partials[i];
-  v = warp_sum(v);
+  double x[kStridedLoads];
+  strided_load(x, partials, count);
+  double v = warp_sum(strided_sum(x));
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
   __syncthreads();
   double r = 0.0;
