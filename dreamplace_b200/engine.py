@@ -156,9 +156,12 @@ class GPEngine(object):
         # theirs by the products' own error (1e-4 of the field of a nearly even
         # density), which 16 iterations of a 200k-cell design turned into up to 6e-3
         # of the gradient, and a run's trajectory is to stay what it was (a solve at
-        # 1024^2 takes 67 us instead of 25); dct_precision "fp32" takes the fast
-        # transforms
-        self.poisson_ws = PoissonWorkspace(ep.num_bins_x, ep.num_bins_y, self.prec, dev, fast=self.prec == 0)
+        # 1024^2 takes 67 us instead of 25); the products' error falls with the square
+        # of the side, and up to 128 bins the fast transforms serve split_bf16 trials
+        # too (28 us -> 10 of a 70 us trial at 128^2); dct_precision "fp32" takes them
+        # at every size they serve
+        fast = self.prec == 0 or (self.prec == 3 and max(ep.num_bins_x, ep.num_bins_y) <= 128)
+        self.poisson_ws = PoissonWorkspace(ep.num_bins_x, ep.num_bins_y, self.prec, dev, fast=fast)
         # spatial visiting order of the scattered cells (movable block, then filler
         # block), refreshed every `sort_interval` iterations (refresh_due)
         nm, nf = d.num_movable_nodes, d.num_filler_nodes
