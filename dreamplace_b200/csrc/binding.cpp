@@ -325,6 +325,15 @@ at::Tensor pin_pos_forward(at::Tensor pos, at::Tensor offx, at::Tensor offy, at:
   c10::cuda::CUDAGuard guard(pos.device());
   int num_pins = offx.numel();
   auto out = at::empty({2 * (int64_t)num_pins}, pos.options());
+  // the interleaved copy costs a pass over the nodes and a launch, and pays
+  // from about a million pins
+  constexpr int kPackPins = 1 << 20;
+  if (num_pins >= kPackPins && num_pins >= pos.numel() / 2) {
+    auto xy = at::empty_like(pos);
+    DP_CALL(dp_pin_pos_forward_xy(ptr<float>(pos), pos.numel() / 2, ptr<float>(offx), ptr<float>(offy),
+                                  ptr<int>(pin2node), num_pins, ptr<float>(xy), ptr<float>(out), cur_stream()));
+    return out;
+  }
   DP_CALL(dp_pin_pos_forward(ptr<float>(pos), pos.numel() / 2, ptr<float>(offx), ptr<float>(offy), ptr<int>(pin2node),
                              num_pins, ptr<float>(out), cur_stream()));
   return out;
@@ -352,6 +361,19 @@ at::Tensor hpwl_forward(at::Tensor pin_pos, at::Tensor flat_netpin, at::Tensor n
                   netpin_start.numel() - 1, net_weights.numel() ? ptr<float>(net_weights) : nullptr,
                   net_mask.data_ptr<uint8_t>(), ptr<double>(out), nullptr, cur_stream()));
   return out.narrow(0, 0, 1);
+}
+
+// the total rounded to fp32, as a scalar
+at::Tensor hpwl_forward_f32(at::Tensor pin_pos, at::Tensor flat_netpin, at::Tensor netpin_start,
+                            at::Tensor net_weights, at::Tensor net_mask) {
+  CHECK_FLAT(pin_pos); CHECK_EVEN(pin_pos); CHECK_F32(pin_pos);
+  c10::cuda::CUDAGuard guard(pin_pos.device());
+  auto buf = at::empty({DP_REDUCE_DOUBLES}, pin_pos.options().dtype(at::kDouble));
+  auto out = at::empty({}, pin_pos.options());
+  DP_CALL(dp_hpwl(ptr<float>(pin_pos), pin_pos.numel() / 2, ptr<int>(flat_netpin), ptr<int>(netpin_start),
+                  netpin_start.numel() - 1, net_weights.numel() ? ptr<float>(net_weights) : nullptr,
+                  net_mask.data_ptr<uint8_t>(), ptr<double>(buf), ptr<float>(out), cur_stream()));
+  return out;
 }
 
 at::Tensor move_boundary_forward(at::Tensor pos, at::Tensor sx, at::Tensor sy, double xl, double yl, double xh,
@@ -638,6 +660,84 @@ void wa_pins_forward(at::Tensor pin_pos, at::Tensor group_deg, at::Tensor group_
                              ptr<float>(grad_lane), cur_stream()));
 }
 
+// value and lane-order gradient with gamma itself (float32 [1]); returns the value as a scalar
+at::Tensor wa_pins_value(at::Tensor pin_pos, at::Tensor group_deg, at::Tensor group_base, at::Tensor group_net,
+                         at::Tensor ln_pin, c10::optional<at::Tensor> net_weights, at::Tensor net_mask,
+                         at::Tensor gamma, at::Tensor grad_lane) {
+  CHECK_FLAT(pin_pos); CHECK_F32(pin_pos); CHECK_EVEN(pin_pos); CHECK_I32(group_deg); CHECK_I32(group_base);
+  CHECK_I32(group_net); CHECK_I32(ln_pin); CHECK_F32(grad_lane); CHECK_F32(gamma); CHECK_CUDA_T(gamma);
+  TORCH_CHECK(group_net.numel() == 32 * group_deg.numel() && group_base.numel() == group_deg.numel(),
+              "wa_pins_value: inconsistent plan");
+  TORCH_CHECK(grad_lane.numel() >= 2 * ln_pin.numel(), "wa_pins_value: grad_lane smaller than the lane slots");
+  TORCH_CHECK(gamma.numel() == 1, "wa_pins_value: gamma must hold one value");
+  auto buf = at::empty({DP_REDUCE_DOUBLES}, pin_pos.options().dtype(at::kDouble));
+  auto out = at::empty({}, pin_pos.options());
+  DP_CALL(dp_wa_pins_value(ptr<float>(pin_pos), pin_pos.numel() / 2, ptr<int>(group_deg), ptr<int>(group_base),
+                           ptr<int>(group_net), group_deg.numel(), ptr<int>(ln_pin), (const float*)ovp(net_weights),
+                           net_mask.data_ptr<uint8_t>(), ptr<float>(gamma), ptr<double>(buf), ptr<float>(grad_lane),
+                           ptr<float>(out), cur_stream()));
+  return out;
+}
+
+// {map, xy_o, overflow f64 [2], overflow f32 [2]} (the last two undefined without overflow)
+std::vector<at::Tensor> density_cells(at::Tensor pos, at::Tensor order, at::Tensor rec4, at::Tensor ratio_o,
+                                      int num_first, int count, at::Tensor init, double xl, double yl, double xh,
+                                      double yh, double bsx, double bsy, int nbx, int nby, int deterministic,
+                                      c10::optional<at::Tensor> scratch, double scale, bool overflow,
+                                      double target_area, double bin_area) {
+  CHECK_FLAT(pos); CHECK_F32(pos); CHECK_EVEN(pos); CHECK_I32(order); CHECK_F32(rec4);
+  CHECK_CUDA_T(init); CHECK_CONTIG(init); CHECK_F32(init);
+  const int64_t nbins = (int64_t)nbx * nby;
+  TORCH_CHECK(order.numel() >= count && 4 * (int64_t)count <= rec4.numel() && count <= ratio_o.numel(),
+              "density_cells: buffers smaller than count");
+  TORCH_CHECK(init.numel() == nbins, "density_cells: the initial map is not num_bins_x*num_bins_y");
+  TORCH_CHECK(!deterministic || (scratch.has_value() && scratch->scalar_type() == at::kLong &&
+                                 scratch->numel() >= nbins),
+              "density_cells: deterministic mode needs an int64 map");
+  c10::cuda::CUDAGuard guard(pos.device());
+  auto out = at::empty({nbx, nby}, pos.options());
+  auto xy_o = at::empty({2 * (int64_t)count}, pos.options());
+  at::Tensor o64, o32;
+  if (overflow) {
+    o64 = at::empty({DP_REDUCE_DOUBLES}, pos.options().dtype(at::kDouble));
+    o32 = at::empty({2}, pos.options());
+  }
+  DP_CALL(dp_density_cells(ptr<float>(pos), pos.numel() / 2, ptr<int>(order), ptr<float>(rec4), ptr<float>(ratio_o),
+                           num_first, count, ptr<float>(init), xl, yl, xh, yh, bsx, bsy, inv_f(bsx), inv_f(bsy), nbx,
+                           nby, deterministic, fraction_bits(xl, yl, xh, yh), (int64_t*)ovp(scratch), (float)scale,
+                           ptr<float>(xy_o), ptr<float>(out), target_area, bin_area,
+                           overflow ? ptr<double>(o64) : nullptr, overflow ? ptr<float>(o32) : nullptr,
+                           cur_stream()));
+  if (!overflow) return {out, xy_o};
+  return {out, xy_o, o64.narrow(0, 0, 2), o32};
+}
+
+at::Tensor electric_force_nodes(at::Tensor grad_pos, at::Tensor ex, at::Tensor ey, at::Tensor xy_o, at::Tensor order,
+                                at::Tensor rec4, at::Tensor ratio_o, int num_movable, int num_filler, int num_nodes,
+                                double xl, double yl, double bsx, double bsy, int nbx, int nby, double scale) {
+  CHECK_FLAT(xy_o); CHECK_F32(xy_o); CHECK_I32(order); CHECK_F32(grad_pos); CHECK_CUDA_T(grad_pos);
+  const int64_t count = (int64_t)num_movable + num_filler;
+  TORCH_CHECK(2 * count <= xy_o.numel() && 4 * count <= rec4.numel() && count <= ratio_o.numel() &&
+                  count <= order.numel(),
+              "electric_force_nodes: buffers smaller than the cells");
+  TORCH_CHECK(ex.numel() == (int64_t)nbx * nby && ey.numel() == ex.numel(), "electric_force_nodes: field map size");
+  auto out = at::empty({2 * (int64_t)num_nodes}, xy_o.options());
+  DP_CALL(dp_electric_force_nodes(ptr<float>(grad_pos), nbx, nby, ptr<float>(ex), ptr<float>(ey), ptr<float>(xy_o),
+                                  ptr<int>(order), ptr<float>(rec4), ptr<float>(ratio_o), num_movable, num_filler,
+                                  num_nodes, xl, yl, bsx, bsy, inv_f(bsx), inv_f(bsy), (float)scale, ptr<float>(out),
+                                  cur_stream()));
+  return out;
+}
+
+void precondition(at::Tensor grad, at::Tensor pws, at::Tensor area, at::Tensor lam, double alpha) {
+  CHECK_CUDA_T(grad); CHECK_CONTIG(grad); CHECK_F32(grad); CHECK_F32(pws); CHECK_F32(area); CHECK_F32(lam);
+  CHECK_CUDA_T(lam); CHECK_CONTIG(pws); CHECK_CONTIG(area);
+  const int64_t n = grad.numel() / 2;
+  TORCH_CHECK(pws.numel() == n && area.numel() == n && lam.numel() == 1, "precondition: size mismatch");
+  DP_CALL(dp_precondition(ptr<float>(grad), ptr<float>(pws), ptr<float>(area), ptr<float>(lam), (float)alpha, (int)n,
+                          cur_stream()));
+}
+
 at::Tensor wa_pins_backward(at::Tensor grad_lane, at::Tensor lane_of_pin, c10::optional<at::Tensor> pin_mask,
                             at::Tensor grad_out) {
   CHECK_F32(grad_lane); CHECK_I32(lane_of_pin); CHECK_F32(grad_out);
@@ -891,6 +991,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("hpwl_forward", &hpwl_forward);
   m.def("move_boundary_forward", &move_boundary_forward);
   m.def("pws_forward", &pws_forward);
+  m.def("hpwl_forward_f32", &hpwl_forward_f32);
+  m.def("wa_pins_value", &wa_pins_value);
+  m.def("density_cells", &density_cells);
+  m.def("electric_force_nodes", &electric_force_nodes);
+  m.def("precondition", &precondition);
   m.def("trial_start", &trial_start);
   m.def("trial_wirelength", &trial_wirelength);
   m.def("trial_density", &trial_density);

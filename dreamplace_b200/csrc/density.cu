@@ -741,6 +741,33 @@ __global__ void __launch_bounds__(256) finish_maps_kernel(MapSums<T> a, int n, d
   block_partial(s, partials);
 }
 
+// out = (init + sum) * scale of one scatter's sums (T as in finish_maps_kernel),
+// with the overflow sum and maximum of init + sum when partials is given
+template <typename T>
+__global__ void __launch_bounds__(256) finish_map_kernel(const T* sum, const float* init, float* out, double inv_scale,
+                                                         float scale, int n, double target_area, double* partials,
+                                                         unsigned* maxkey) {
+  grid_dep_sync();
+  double s = 0.0;
+  float m = -INFINITY;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const float in = init ? init[i] : 0.f;
+    float d;
+    if constexpr (std::is_same<T, float>::value)
+      d = fadd(in, sum[i]);
+    else
+      d = (float)((double)in + (double)sum[i] * inv_scale);
+    out[i] = fmul(d, scale);
+    const double over = (double)d - target_area;
+    s += over > 0.0 ? over : 0.0;
+    m = fmaxf(m, d);
+  }
+  if (!partials) return;  // uniform: no overflow wanted
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(maxkey, float_key(m));
+  block_partial(s, partials);
+}
+
 __global__ void overflow_finish_kernel(double* out2, const unsigned* maxkey, double bin_area,
                                        float* out2_f32, const double* partials, int count) {
   grid_dep_sync();
@@ -1406,13 +1433,31 @@ __global__ void order_place_kernel(const unsigned* __restrict__ keys, int num_no
   }
 }
 
-// xy_o[idx] = (x, y) of node order[idx], from planar positions [x(n) | y(n)]
-__global__ void gather_order_pos_kernel(const float* __restrict__ pos, int num_nodes, const int* __restrict__ order,
-                                        int count, float2* __restrict__ xy_o) {
+// xy_o[idx] = (x, y) of node order[idx], from planar positions [x(n) | y(n)];
+// four cells of a thread in flight.  zero (optional): the words that the
+// scatter behind it adds into, and its overflow's key
+__global__ void __launch_bounds__(256) gather_order_pos_kernel(const float* __restrict__ pos, int num_nodes,
+                                                               const int* __restrict__ order, int count,
+                                                               float2* __restrict__ xy_o, uint32_t* __restrict__ zero,
+                                                               long long zero_words, double* __restrict__ zero_cell) {
   grid_dep_sync();
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-    const int i = __ldg(order + idx);
-    xy_o[idx] = make_float2(__ldg(pos + i), __ldg(pos + num_nodes + i));
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  for (long long i = tid; i < zero_words; i += stride) zero[i] = 0u;
+  if (zero_cell && tid == 0) *zero_cell = 0.0;
+  for (int idx = tid; idx < count; idx += 4 * stride) {
+    int o[4];
+    float2 q[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long k = idx + (long long)u * stride;
+      o[u] = k < count ? __ldg(order + k) : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (o[u] >= 0) q[u] = make_float2(__ldg(pos + o[u]), __ldg(pos + num_nodes + o[u]));
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (o[u] >= 0) xy_o[idx + (long long)u * stride] = q[u];
   }
 }
 
@@ -1482,6 +1527,58 @@ extern "C" int dp_gather_order_pos(const float* pos, int num_nodes, const int* o
   DP_REQUIRE(((uintptr_t)xy_o & 7) == 0, "dp_gather_order_pos: xy_o must be 8-byte aligned");
   if (count == 0) return DP_OK;
   launch_kernel(gather_order_pos_kernel, grid_for(count, 256, 8), 256, 0, as_stream(stream), 
-      pos, num_nodes, order, count, reinterpret_cast<float2*>(xy_o));
+      pos, num_nodes, order, count, reinterpret_cast<float2*>(xy_o), (uint32_t*)nullptr, 0ll, (double*)nullptr);
   return check_launch("dp_gather_order_pos");
+}
+
+// The density map of a module's cells in three launches (four with the
+// overflow): the gather into visiting order, which also zeroes the sums; one
+// scatter of both ranges onto one map; and a pass that adds the initial map,
+// scales, and reduces the overflow.  The calls it replaces (a memset, scatter
+// and conversion for each range, the scaling, the overflow's own passes) were
+// up to eleven, and a module call on fewer than ~100k cells is bound by them.
+extern "C" int dp_density_cells(const float* pos, int num_nodes, const int* order, const float* rec4,
+                                const float* ratio_o, int num_first, int count, const float* init, float xl, float yl,
+                                float xh, float yh, float bsx, float bsy, float ibx, float iby, int nbx, int nby,
+                                int deterministic, int fraction_bits, int64_t* scratch, float scale, float* xy_o,
+                                float* out, double target_area, double bin_area, double* overflow_out,
+                                float* overflow_f32, dp_stream_t stream) {
+  using namespace dpb;
+  OrderedScatter o;
+  int rc = ordered_setup("dp_density_cells", xy_o, nullptr, rec4, ratio_o, count, xl, yl, bsx, bsy, ibx, iby, nbx, nby,
+                         deterministic, fraction_bits, scratch, stream, o);
+  if (rc) return rc;
+  DP_REQUIRE(pos && (order || count == 0) && out, "dp_density_cells: null pointer argument");
+  DP_REQUIRE(num_first >= 0 && num_first <= count, "dp_density_cells: bad num_first");
+  DP_REQUIRE(!overflow_out || bin_area > 0, "dp_density_cells: bad bin area");
+  const int nbins = nbx * nby;
+  double* cell = overflow_out ? overflow_out + 2 : nullptr;
+  const long long words = (long long)nbins * (deterministic ? 2 : 1);
+  launch_kernel(gather_order_pos_kernel, grid_for(count > nbins ? count : nbins, 256, 8), 256, 0, o.s, pos, num_nodes,
+                order, count, reinterpret_cast<float2*>(xy_o), deterministic ? (uint32_t*)scratch : (uint32_t*)out,
+                words, cell);
+  rc = check_launch("dp_density_cells gather");
+  if (rc) return rc;
+  WsRanges rg;
+  memset(&rg, 0, sizeof(rg));
+  rg.b1 = num_first;
+  rg.b2 = count;
+  rg.map0_f32 = rg.map1_f32 = out;
+  rg.map0_fx = rg.map1_fx = reinterpret_cast<unsigned long long*>(scratch);
+  rc = scatter_ranges(o, rg, deterministic, fraction_bits);
+  if (rc) return rc;
+  const int blocks = grid_for(nbins, 256, 4);
+  double* partials = overflow_out ? overflow_out + 3 : nullptr;
+  unsigned* key = reinterpret_cast<unsigned*>(cell);
+  if (deterministic)
+    launch_kernel(finish_map_kernel<long long>, blocks, 256, 0, o.s, (const long long*)scratch, init, out,
+                  ldexp(1.0, -fraction_bits), scale, nbins, target_area, partials, key);
+  else
+    launch_kernel(finish_map_kernel<float>, blocks, 256, 0, o.s, (const float*)out, init, out, 0.0, scale, nbins,
+                  target_area, partials, key);
+  rc = check_launch("dp_density_cells finish");
+  if (rc || !overflow_out) return rc;
+  launch_kernel(overflow_finish_kernel, 1, kReduceThreads, 0, o.s, overflow_out, key, bin_area, overflow_f32, partials,
+                blocks);
+  return check_launch("dp_density_cells overflow");
 }

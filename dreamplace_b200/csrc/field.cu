@@ -72,11 +72,19 @@ struct ForceScale {
   const float* factor_quad;
 };
 
+// where the force goes in node order (out null: order space instead), and the
+// nodes between the movable cells and the fillers, whose force is zero
+struct ForceNodes {
+  float* out;
+  const int* order;
+  int num_nodes, zero_begin, zero_end;
+};
+
 __global__ void __launch_bounds__(256) electric_force_records_kernel(
     ForceScale fs, int nbx, int nby, const float* __restrict__ ex, const float* __restrict__ ey,
     const float2* __restrict__ xy_o, const int* __restrict__ order, const float4* __restrict__ rec4,
     const float* __restrict__ ratio_o, int count, float xl, float yl, float bsx, float bsy, float ibx, float iby,
-    float scale, float2* __restrict__ force_o, const int* __restrict__ gate) {
+    float scale, float2* __restrict__ force_o, ForceNodes nodes, const int* __restrict__ gate) {
   grid_dep_sync();
   if (gate_closed(gate)) return;
   const float g = fs.grad_pos ? fs.grad_pos[0] : objective_grad_scale(fs.energy[0], fs.density_weight, fs.factor_quad);
@@ -126,27 +134,43 @@ __global__ void __launch_bounds__(256) electric_force_records_kernel(
       }
     }
     const float r = __ldcs(ratio_o + idx);
-    force_o[idx] = make_float2(fmul(fmul(fmul(gx, r), g), scale), fmul(fmul(fmul(gy, r), g), scale));
+    gx = fmul(fmul(fmul(gx, r), g), scale);
+    gy = fmul(fmul(fmul(gy, r), g), scale);
+    if (nodes.out) {
+      // scattered words, which L2 merges: a pass of its own that put the pairs
+      // back in node order took 34 us of the 3.1M cells' 73
+      const int i = __ldg(nodes.order + idx);
+      nodes.out[i] = gx;
+      nodes.out[nodes.num_nodes + i] = gy;
+    } else {
+      force_o[idx] = make_float2(gx, gy);
+    }
   }
+  if (nodes.out)
+    for (int i = nodes.zero_begin + blockIdx.x * blockDim.x + threadIdx.x; i < nodes.zero_end;
+         i += gridDim.x * blockDim.x) {
+      nodes.out[i] = 0.f;
+      nodes.out[nodes.num_nodes + i] = 0.f;
+    }
 }
 
 }  // namespace dpb
 
 using namespace dpb;
 
-static int force_ordered(const ForceScale& fs, int nbx, int nby, const float* ex, const float* ey,
+static int force_ordered(const ForceScale& fs, const ForceNodes& nodes, int nbx, int nby, const float* ex, const float* ey,
                                          const float* xy_o, const int* order, const float* rec4,
                                          const float* ratio_o,
                                          int count, float xl, float yl, float bsx, float bsy, float ibx, float iby,
                                          float scale, float* force_o, dp_stream_t stream) {
-  DP_REQUIRE(ex && ey && xy_o && rec4 && ratio_o && force_o,
+  DP_REQUIRE(ex && ey && xy_o && rec4 && ratio_o && (force_o || nodes.out),
              "dp_electric_force_ordered: null pointer argument");
   DP_REQUIRE(((uintptr_t)xy_o & 7) == 0 && ((uintptr_t)rec4 & 15) == 0 && ((uintptr_t)force_o & 7) == 0,
              "dp_electric_force_ordered: misaligned xy_o / rec4 / force_o");
-  if (count == 0) return DP_OK;
+  if (count == 0 && !(nodes.out && nodes.zero_end > nodes.zero_begin)) return DP_OK;
   launch_kernel(electric_force_records_kernel, grid_for(count, 256, 16), 256, 0, as_stream(stream), 
       fs, nbx, nby, ex, ey, reinterpret_cast<const float2*>(xy_o), order, reinterpret_cast<const float4*>(rec4),
-      ratio_o, count, xl, yl, bsx, bsy, ibx, iby, scale, reinterpret_cast<float2*>(force_o), trial_gate());
+      ratio_o, count, xl, yl, bsx, bsy, ibx, iby, scale, reinterpret_cast<float2*>(force_o), nodes, trial_gate());
   return check_launch("dp_electric_force_ordered");
 }
 
@@ -157,8 +181,22 @@ extern "C" int dp_electric_force_ordered(const float* grad_pos, int nbx, int nby
                                          float scale, float* force_o, dp_stream_t stream) {
   DP_REQUIRE(grad_pos, "dp_electric_force_ordered: null pointer argument");
   const ForceScale fs = {grad_pos, nullptr, nullptr, nullptr};
-  return force_ordered(fs, nbx, nby, ex, ey, xy_o, order, rec4, ratio_o, count, xl, yl, bsx, bsy, ibx, iby, scale,
+  return force_ordered(fs, ForceNodes(), nbx, nby, ex, ey, xy_o, order, rec4, ratio_o, count, xl, yl, bsx, bsy, ibx, iby, scale,
                        force_o, stream);
+}
+
+extern "C" int dp_electric_force_nodes(const float* grad_pos, int nbx, int nby, const float* ex, const float* ey,
+                                       const float* xy_o, const int* order, const float* rec4, const float* ratio_o,
+                                       int num_movable, int num_filler, int num_nodes, float xl, float yl, float bsx,
+                                       float bsy, float ibx, float iby, float scale, float* out,
+                                       dp_stream_t stream) {
+  DP_REQUIRE(grad_pos && order && out, "dp_electric_force_nodes: null pointer argument");
+  DP_REQUIRE(num_movable >= 0 && num_filler >= 0 && num_movable + num_filler <= num_nodes,
+             "dp_electric_force_nodes: bad node counts");
+  const ForceScale fs = {grad_pos, nullptr, nullptr, nullptr};
+  const ForceNodes nodes = {out, order, num_nodes, num_movable, num_nodes - num_filler};
+  return force_ordered(fs, nodes, nbx, nby, ex, ey, xy_o, nullptr, rec4, ratio_o, num_movable + num_filler, xl, yl, bsx,
+                       bsy, ibx, iby, scale, nullptr, stream);
 }
 
 extern "C" int dp_trial_force(const double* energy, const float* density_weight, const float* factor_quad, int nbx, int nby, const float* ex, const float* ey,
@@ -168,7 +206,7 @@ extern "C" int dp_trial_force(const double* energy, const float* density_weight,
                                          float scale, float* force_o, dp_stream_t stream) {
   DP_REQUIRE(energy && density_weight && factor_quad, "dp_trial_force: null pointer argument");
   const ForceScale fs = {nullptr, energy, density_weight, factor_quad};
-  return force_ordered(fs, nbx, nby, ex, ey, xy_o, order, rec4, ratio_o, count, xl, yl, bsx, bsy, ibx, iby, scale,
+  return force_ordered(fs, ForceNodes(), nbx, nby, ex, ey, xy_o, order, rec4, ratio_o, count, xl, yl, bsx, bsy, ibx, iby, scale,
                        force_o, stream);
 }
 

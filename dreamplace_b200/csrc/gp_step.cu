@@ -448,6 +448,32 @@ extern "C" int dp_precondition_step_size(float* g_new, const float* g, const flo
   return check_launch("dp_precondition_step_size finish");
 }
 
+namespace dpb {
+// grad /= max(1, pws + (alpha lambda) area), the order and rounding of the
+// reference's tensor expression (a NaN preconditioner stays NaN, as clamp keeps it)
+__global__ void __launch_bounds__(256) precondition_kernel(float* __restrict__ grad, const float* __restrict__ pws,
+                                                           const float* __restrict__ area,
+                                                           const float* __restrict__ lam_p, float alpha, int n) {
+  grid_dep_sync();
+  const float lam = fmul(alpha, *lam_p);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    float p = fadd(pws[i], fmul(lam, area[i]));
+    if (p < 1.0f) p = 1.0f;
+    grad[i] = __fdiv_rn(grad[i], p);
+    grad[i + n] = __fdiv_rn(grad[i + n], p);
+  }
+}
+}  // namespace dpb
+
+extern "C" int dp_precondition(float* grad, const float* pws, const float* area, const float* lambda_, float alpha,
+                               int num_nodes, dp_stream_t stream) {
+  DP_REQUIRE(grad && pws && area && lambda_ && num_nodes >= 0, "dp_precondition: bad arguments");
+  if (num_nodes == 0) return DP_OK;
+  launch_kernel(precondition_kernel, grid_for(num_nodes, 256, 8), 256, 0, as_stream(stream), grad, pws, area, lambda_,
+                alpha, num_nodes);
+  return check_launch("dp_precondition");
+}
+
 // What the GP loop does on the host between iteration k and k+1, on the
 // device, so that iteration k+1 can be enqueued before the host has read
 // iteration k's metrics:
@@ -753,6 +779,7 @@ struct LaneArgs {
   const unsigned char* net_mask;
   const unsigned char* hpwl_mask;
   const float* inv_gamma;  // device scalar (read once per thread)
+  bool is_gamma;           // the scalar is gamma itself
   float2* gnode;
 };
 
@@ -1109,7 +1136,7 @@ __global__ void __launch_bounds__(256, 4) wa_lane_kernel(LaneArgs A, double* __r
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const bool hpwl = kGrad && hpwl_partials != nullptr;
-  const float ig = kGrad ? *A.inv_gamma : 0.f;
+  const float ig = kGrad ? (A.is_gamma ? __fdiv_rn(1.0f, *A.inv_gamma) : *A.inv_gamma) : 0.f;
   double contrib = 0.0, hcontrib = 0.0;
   for (int g = warp; g < A.num_groups; g += nwarps) {
     const int deg = A.group_deg[g], base = A.group_base[g];
@@ -1239,7 +1266,7 @@ extern "C" int dp_plan_net_lanes(const int* netpin_start_host, int num_nets, con
 
 // blocks_out given: the partials are left for a later finisher, which gets their count
 static int launch_lanes(bool grad, const dpb::LaneArgs& A, double* out_f64, double* hpwl_f64, cudaStream_t s,
-                        int* blocks_out = nullptr) {
+                        int* blocks_out = nullptr, float* out_f32 = nullptr) {
   using namespace dpb;
   // one wave: the launch bounds keep 4 blocks of 256 resident per SM, and the
   // warps stride over the groups, so a larger grid only adds a partial last
@@ -1262,7 +1289,7 @@ static int launch_lanes(bool grad, const dpb::LaneArgs& A, double* out_f64, doub
   }
   // the WA total and the HPWL (same fixed-order reduction each) in one launch
   if (grad && hpwl_f64) return launch_finish_sum2(out_f64, hpwl_f64, blocks, s);
-  return launch_finish_sum(out_f64, blocks, nullptr, s);
+  return launch_finish_sum(out_f64, blocks, out_f32, s);
 }
 
 static dpb::LaneArgs lane_args(const float* xy, const int* group_deg, const int* group_base, const int* group_net,
@@ -1284,6 +1311,7 @@ static dpb::LaneArgs lane_args(const float* xy, const int* group_deg, const int*
   A.net_mask = net_mask;
   A.hpwl_mask = hpwl_mask;
   A.inv_gamma = inv_gamma;
+  A.is_gamma = false;
   A.gnode = reinterpret_cast<float2*>(grad_node_order);
   return A;
 }
@@ -1342,10 +1370,10 @@ extern "C" int dp_hpwl_lanes(const float* xy, const int* group_deg, const int* g
 // The lane-per-net WA of dp_wa_lanes_forward reading the pins' own positions
 // (planar [x(P) | y(P)], the layout of the reference op's input), for the
 // drop-in WeightedAverageWirelength: the lane slots hold pin ids.
-extern "C" int dp_wa_pins_forward(const float* pin_pos, int num_pins, const int* group_deg, const int* group_base,
+static int wa_pins(const float* pin_pos, int num_pins, const int* group_deg, const int* group_base,
                                   const int* group_net, int num_groups, const int* ln_pin, const float* net_weights,
                                   const unsigned char* net_mask, const float* inv_gamma, double* wl_f64,
-                                  float* grad_lane, dp_stream_t stream) {
+                                  float* grad_lane, bool is_gamma, float* wl_f32, dp_stream_t stream) {
   DP_REQUIRE(pin_pos && group_deg && group_base && group_net && ln_pin && net_mask && inv_gamma && wl_f64 && grad_lane,
              "dp_wa_pins_forward: null pointer argument");
   DP_REQUIRE(num_pins >= 0 && num_groups >= 0, "dp_wa_pins_forward: bad sizes");
@@ -1354,7 +1382,28 @@ extern "C" int dp_wa_pins_forward(const float* pin_pos, int num_pins, const int*
                               net_weights, net_mask, nullptr, inv_gamma, grad_lane);
   A.px = pin_pos;
   A.py = pin_pos + num_pins;
-  return launch_lanes(true, A, wl_f64, nullptr, dpb::as_stream(stream));
+  A.is_gamma = is_gamma;
+  return launch_lanes(true, A, wl_f64, nullptr, dpb::as_stream(stream), nullptr, wl_f32);
+}
+
+extern "C" int dp_wa_pins_forward(const float* pin_pos, int num_pins, const int* group_deg, const int* group_base,
+                                  const int* group_net, int num_groups, const int* ln_pin, const float* net_weights,
+                                  const unsigned char* net_mask, const float* inv_gamma, double* wl_f64,
+                                  float* grad_lane, dp_stream_t stream) {
+  return wa_pins(pin_pos, num_pins, group_deg, group_base, group_net, num_groups, ln_pin, net_weights, net_mask, inv_gamma,
+                 wl_f64, grad_lane, false, nullptr, stream);
+}
+
+// gamma instead of its reciprocal, and the value also as a float: three one-element
+// kernels fewer on each call of the module, which is bound by its launches up to ~100k cells
+extern "C" int dp_wa_pins_value(const float* pin_pos, int num_pins, const int* group_deg, const int* group_base,
+                                  const int* group_net, int num_groups, const int* ln_pin, const float* net_weights,
+                                  const unsigned char* net_mask, const float* gamma, double* wl_f64,
+                                  float* grad_lane, float* wl_f32,
+                                  dp_stream_t stream) {
+  DP_REQUIRE(wl_f32, "dp_wa_pins_value: null pointer argument");
+  return wa_pins(pin_pos, num_pins, group_deg, group_base, group_net, num_groups, ln_pin, net_weights, net_mask, gamma,
+                 wl_f64, grad_lane, true, wl_f32, stream);
 }
 
 namespace dpb {

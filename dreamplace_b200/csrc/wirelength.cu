@@ -124,10 +124,12 @@ __global__ void wa_merged_backward_kernel(const float* __restrict__ grad_pos,
 }
 
 // Four pins of a thread in flight: pin -> node -> position is a chain of two
-// dependent reads, so the time is theirs, not the bytes'.  MEASURED_PPF
+// dependent reads.  Each read of a node position moves a 32-byte sector of L2
+// for 4 bytes; through an interleaved copy (kXY) both coordinates come in one.
+template <bool kXY>
 __global__ void __launch_bounds__(256) pin_pos_forward_kernel(
-    const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ offx,
-    const float* __restrict__ offy, const int* __restrict__ pin2node, int num_pins, float* __restrict__ pin_x,
+    const float* __restrict__ x, const float* __restrict__ y, const float2* __restrict__ xy,
+    const float* __restrict__ offx, const float* __restrict__ offy, const int* __restrict__ pin2node, int num_pins, float* __restrict__ pin_x,
     float* __restrict__ pin_y) {
   grid_dep_sync();
   const int stride = gridDim.x * blockDim.x;
@@ -139,8 +141,9 @@ __global__ void __launch_bounds__(256) pin_pos_forward_kernel(
     for (int u = 0; u < 4; ++u) n[u] = __ldcs(pin2node + p + u * stride);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      vx[u] = x[n[u]];
-      vy[u] = y[n[u]];
+      const float2 q = kXY ? __ldg(xy + n[u]) : make_float2(__ldg(x + n[u]), __ldg(y + n[u]));
+      vx[u] = q.x;
+      vy[u] = q.y;
       ox[u] = __ldcs(offx + p + u * stride);
       oy[u] = __ldcs(offy + p + u * stride);
     }
@@ -152,8 +155,9 @@ __global__ void __launch_bounds__(256) pin_pos_forward_kernel(
   }
   for (; p < num_pins; p += stride) {
     const int n = pin2node[p];
-    pin_x[p] = fadd(offx[p], x[n]);
-    pin_y[p] = fadd(offy[p], y[n]);
+    const float2 q = kXY ? __ldg(xy + n) : make_float2(__ldg(x + n), __ldg(y + n));
+    pin_x[p] = fadd(offx[p], q.x);
+    pin_y[p] = fadd(offy[p], q.y);
   }
 }
 
@@ -190,7 +194,6 @@ __device__ __forceinline__ void warp_fold(float2* stage, const int* __restrict__
   }
 }
 
-// MEASURED_PPB
 __global__ void __launch_bounds__(kFoldThreads) pin_pos_backward_kernel(
     const float* __restrict__ gpx, const float* __restrict__ gpy, const int* __restrict__ flat_node2pin,
     const int* __restrict__ node_start, int num_physical, int num_nodes, float* __restrict__ gx,
@@ -218,7 +221,6 @@ __global__ void __launch_bounds__(kFoldThreads) pin_pos_backward_kernel(
   }
 }
 
-// MEASURED_HPWL
 __global__ void __launch_bounds__(kFoldThreads) hpwl_kernel(const float* __restrict__ px, const float* __restrict__ py,
                                                             const int* __restrict__ flat_netpin,
                                                             const int* __restrict__ netpin_start, int num_nets,
@@ -324,9 +326,22 @@ extern "C" int dp_pin_pos_forward(const float* pos, int num_nodes, const float* 
                                   float* pin_pos, dp_stream_t stream) {
   DP_REQUIRE(pos && offx && offy && pin2node && pin_pos, "dp_pin_pos_forward: null pointer argument");
   if (num_pins == 0) return DP_OK;
-  launch_kernel(pin_pos_forward_kernel, grid_for(num_pins, 256, 8), 256, 0, as_stream(stream), 
-      pos, pos + num_nodes, offx, offy, pin2node, num_pins, pin_pos, pin_pos + num_pins);
+  launch_kernel(pin_pos_forward_kernel<false>, grid_for(num_pins, 256, 8), 256, 0, as_stream(stream), 
+      pos, pos + num_nodes, (const float2*)nullptr, offx, offy, pin2node, num_pins, pin_pos, pin_pos + num_pins);
   return check_launch("dp_pin_pos_forward");
+}
+
+extern "C" int dp_pin_pos_forward_xy(const float* pos, int num_nodes, const float* offx, const float* offy,
+                                     const int* pin2node, int num_pins, float* xy_work, float* pin_pos,
+                                     dp_stream_t stream) {
+  DP_REQUIRE(pos && offx && offy && pin2node && pin_pos && xy_work, "dp_pin_pos_forward_xy: null pointer argument");
+  if (num_pins == 0) return DP_OK;
+  int rc = dp_pack_xy(pos, num_nodes, xy_work, stream);
+  if (rc) return rc;
+  launch_kernel(pin_pos_forward_kernel<true>, grid_for(num_pins, 256, 8), 256, 0, as_stream(stream), 
+      pos, pos + num_nodes, reinterpret_cast<const float2*>(xy_work), offx, offy, pin2node, num_pins, pin_pos,
+      pin_pos + num_pins);
+  return check_launch("dp_pin_pos_forward_xy");
 }
 
 extern "C" int dp_pin_pos_backward(const float* grad_pin, int num_pins, const int* flat_node2pin,

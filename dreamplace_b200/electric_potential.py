@@ -230,11 +230,17 @@ def poisson_solve(rho, bin_size_x, bin_size_y, precision, fast_mode=False, rho_s
     return ex, ey, energy
 
 
-def _fast_solve(precision, deterministic):
-    """Whether a density operator's solve may take the fast transforms: not a
-    split_bf16 one, whose products' own error (up to 1e-3 of the field of a nearly
-    even density) would show between the two."""
-    return precision_code(precision) != 3
+FAST_SPLIT_SIDE = 512
+
+
+def _fast_solve(precision, rho):
+    """Whether a density operator's solve may take the fast transforms: a
+    split_bf16 one up to 512 bins a side.  The products' own error grows with the
+    grid (of the field of a nearly even density 5e-6 at 64 bins, 2e-5 at 256, up
+    to 1e-3 at 1024, where it would show between the two); the fast transforms'
+    is 1e-7, and a call of the products is 5 launches and 10 allocations against
+    3 and 4."""
+    return precision_code(precision) != 3 or max(rho.shape) <= FAST_SPLIT_SIDE
 
 
 class ElectricDensityMapFunction(Function):
@@ -300,15 +306,20 @@ class CellOrder(object):
                              order, self.count, rec4, ratio_o, None)
         self.order, self.rec4, self.ratio_o = order, rec4, ratio_o
 
-    def positions(self, pos):
-        """The cells' positions in visiting order (interleaved), refreshing the
-        order when due; returns (xy_o, order, rec4, ratio_o)."""
+    def due(self, pos):
+        """Counts a call and refreshes the order when due; returns (order, rec4, ratio_o)."""
         if self.order is None or (self.interval > 0 and self.calls % self.interval == 0):
             self._refresh(pos)
         self.calls += 1
+        return self.order, self.rec4, self.ratio_o
+
+    def positions(self, pos):
+        """The cells' positions in visiting order (interleaved), refreshing the
+        order when due; returns (xy_o, order, rec4, ratio_o)."""
+        order, rec4, ratio_o = self.due(pos)
         xy_o = torch.empty(2 * self.count, dtype=torch.float32, device=pos.device)
-        C.gather_order_pos(pos, self.order, self.count, xy_o)
-        return xy_o, self.order, self.rec4, self.ratio_o
+        C.gather_order_pos(pos, order, self.count, xy_o)
+        return xy_o, order, rec4, ratio_o
 
 
 class ElectricOverflow(nn.Module):
@@ -388,35 +399,36 @@ class ElectricOverflow(nn.Module):
             self._fixed_scratch = torch.empty(self.num_bins_x * self.num_bins_y, dtype=torch.int64, device=device)
         return self._fixed_scratch
 
-    def ordered_density_map(self, pos, num_filler_nodes):
+    def ordered_density_map(self, pos, num_filler_nodes, scale=1.0, overflow=False):
         """The density map of the movable cells and num_filler_nodes fillers on
-        the initial map, by the order-driven scatter (window kernel, block-local
-        sort, shared-memory tiles): the same map as ElectricDensityMapFunction
-        (bit for bit in deterministic mode), with the padding bins filled.
-        Returns (density_map [M, N], (xy_o, order, rec4, ratio_o))."""
+        the initial map, by the order-driven scatter (dp_density_cells): the same
+        map as ElectricDensityMapFunction (bit for bit in deterministic mode),
+        with the padding bins filled, times ``scale``.  Returns
+        (density_map [M, N], (xy_o, order, rec4, ratio_o)), and with ``overflow``
+        also (overflow, max density) of the unscaled map in fp64 and in fp32."""
         require_cuda(pos, "pos")
-        cells = self.cell_order(num_filler_nodes).positions(pos.view(pos.numel()))
-        xy_o, order, rec4, ratio_o = cells
+        pos = pos.view(pos.numel())
+        order, rec4, ratio_o = self.cell_order(num_filler_nodes).due(pos)
         M, N = self.num_bins_x, self.num_bins_y
         det = int(bool(self.deterministic_flag))
-        scratch = self.fixed_scratch(pos.device) if det else None
-        geo = (float(self.xl), float(self.yl), float(self.xh), float(self.yh), float(self.bin_size_x),
-               float(self.bin_size_y), M, N)
-        out = torch.empty(M * N, dtype=torch.float32, device=pos.device)
         nm = self.num_movable_nodes
-        count = nm + num_filler_nodes
-        if num_filler_nodes > 0 and nm > 0:
-            # movable cells block-sorted, fillers (about one per bin) not
-            first = torch.empty_like(out)
-            C.density_map_ordered_split(xy_o, rec4, ratio_o, nm, count, self.initial_density_map.view(-1), *geo, det,
-                                        scratch, first, out, 1.0, 1.0, None)
-        else:
-            C.density_map_ordered_into(xy_o, rec4, ratio_o, count, self.initial_density_map.view(-1), *geo, det,
-                                       scratch, out)
-        density_map = out.view(M, N)
-        if self.padding > 0:
-            density_map.masked_fill_(self.padding_mask, self.target_density * self.bin_size_x * self.bin_size_y)
-        return density_map, cells
+        bin_area = self.bin_size_x * self.bin_size_y
+        padded = self.padding > 0
+        out = C.density_cells(pos, order, rec4, ratio_o, nm, nm + num_filler_nodes, self.initial_density_map,
+                              float(self.xl), float(self.yl), float(self.xh), float(self.yh),
+                              float(self.bin_size_x), float(self.bin_size_y), M, N, det,
+                              self.fixed_scratch(pos.device) if det else None, 1.0 if padded else float(scale),
+                              overflow and not padded, float(self.target_density * bin_area), float(bin_area))
+        density_map, cells = out[0], (out[1], order, rec4, ratio_o)
+        ovf = tuple(out[2:])
+        if padded:
+            density_map.masked_fill_(self.padding_mask, self.target_density * bin_area)
+            if overflow:
+                o64 = C.density_overflow(density_map, float(self.target_density * bin_area), float(bin_area))
+                ovf = (o64, o64.float())
+            if scale != 1.0:
+                density_map.mul_(scale)
+        return (density_map, cells, ovf) if overflow else (density_map, cells)
 
     def compute_initial_density_map(self, pos):
         """Fixed-cell map ×target_density (reference electric_overflow.py:229-258)."""
@@ -448,13 +460,13 @@ class ElectricOverflow(nn.Module):
         """(overflow, max_density) accumulated in fp64, as a [2] float64 tensor."""
         if self.initial_density_map is None:
             self.compute_initial_density_map(pos)
-        density_map, _ = self.ordered_density_map(pos, self.num_filler_nodes)
-        bin_area = self.bin_size_x * self.bin_size_y
-        return C.density_overflow(density_map, float(self.target_density * bin_area), float(bin_area))
+        return self.ordered_density_map(pos, self.num_filler_nodes, overflow=True)[2][0]
 
     def forward(self, pos):
-        out = self.overflow_f64(pos)
-        return out[0:1].float(), out[1:2].float()
+        if self.initial_density_map is None:
+            self.compute_initial_density_map(pos)
+        out = self.ordered_density_map(pos, self.num_filler_nodes, overflow=True)[2][1]
+        return out[0:1], out[1:2]
 
 
 class ElectricPotentialFunction(Function):
@@ -490,11 +502,11 @@ class ElectricPotentialFunction(Function):
             # keep only rho; the backward recomputes the field maps
             energy = torch.zeros(1, dtype=torch.float64, device=pos.device) if fast_mode else \
                 poisson_energy(density_map, bin_size_x, bin_size_y, precision,
-                               _fast_solve(precision, deterministic_flag))
+                               _fast_solve(precision, density_map))
             ctx.field_map_x = ctx.field_map_y = None
         else:
             ex, ey, energy = poisson_solve(density_map, bin_size_x, bin_size_y, precision, fast_mode,
-                                           fast=_fast_solve(precision, deterministic_flag))
+                                           fast=_fast_solve(precision, density_map))
             ctx.field_map_x = ex
             ctx.field_map_y = ey
         if fast_mode:
@@ -510,7 +522,7 @@ class ElectricPotentialFunction(Function):
         fx, fy = ctx.field_map_x, ctx.field_map_y
         if fx is None:
             fx, fy, _ = poisson_solve(ctx.density_map, bsx, bsy, ctx.precision, True,
-                                      fast=_fast_solve(ctx.precision, ctx.deterministic_flag))
+                                      fast=_fast_solve(ctx.precision, ctx.density_map))
         output = C.electric_force(g, nbx, nby, a, b, c, d, fx.view([-1]), fy.view([-1]),
                                   ctx.pos, sxc, syc, ox, oy, ratio, bcx, bcy, float(xl), float(yl), float(xh),
                                   float(yh), float(bsx), float(bsy), int(nm), int(nf),
@@ -521,25 +533,24 @@ class ElectricPotentialFunction(Function):
 class ElectricPotentialOrderedFunction(Function):
     """ElectricPotentialFunction over a visiting order: the order-driven
     scatter in forward and the order-driven field gather in backward
-    (dp_electric_force_ordered), whose force is put back in node order; the
+    (dp_electric_force_nodes), which writes the force in node order; the
     same results as ElectricPotentialFunction (bit for bit in deterministic
     mode)."""
 
     @staticmethod
     def forward(ctx, pos, op, precision, fast_mode, recompute_field):
-        density_map, cells = op.ordered_density_map(pos, op.num_filler_nodes)
         bsx, bsy = op.bin_size_x, op.bin_size_y
-        density_map.mul_(1.0 / (bsx * bsy))
+        density_map, cells = op.ordered_density_map(pos, op.num_filler_nodes, 1.0 / (bsx * bsy))
         ctx.op, ctx.cells, ctx.precision = op, cells, precision
         ctx.num_nodes = pos.numel() // 2
         ctx.density_map = density_map
         if recompute_field:
             energy = torch.zeros(1, dtype=torch.float64, device=pos.device) if fast_mode else \
-                poisson_energy(density_map, bsx, bsy, precision, _fast_solve(precision, op.deterministic_flag))
+                poisson_energy(density_map, bsx, bsy, precision, _fast_solve(precision, density_map))
             ctx.field_map_x = ctx.field_map_y = None
         else:
             ex, ey, energy = poisson_solve(density_map, bsx, bsy, precision, fast_mode,
-                                           fast=_fast_solve(precision, op.deterministic_flag))
+                                           fast=_fast_solve(precision, density_map))
             ctx.field_map_x, ctx.field_map_y = ex, ey
         if fast_mode:
             return torch.zeros(1, dtype=pos.dtype, device=pos.device)
@@ -549,17 +560,15 @@ class ElectricPotentialOrderedFunction(Function):
     def backward(ctx, grad_pos):
         op = ctx.op
         xy_o, order, rec4, ratio_o = ctx.cells
-        count = order.numel()
         fx, fy = ctx.field_map_x, ctx.field_map_y
         if fx is None:
             fx, fy, _ = poisson_solve(ctx.density_map, op.bin_size_x, op.bin_size_y, ctx.precision, True,
-                                      fast=_fast_solve(ctx.precision, op.deterministic_flag))
+                                      fast=_fast_solve(ctx.precision, ctx.density_map))
         g = grad_pos.reshape(1).to(torch.float32)
-        force_o = torch.empty(2 * count, dtype=torch.float32, device=g.device)
-        C.electric_force_ordered(g, fx.view(-1), fy.view(-1), xy_o, rec4, ratio_o, count, float(op.xl), float(op.yl),
-                                 float(op.bin_size_x), float(op.bin_size_y), op.num_bins_x, op.num_bins_y, -1.0,
-                                 force_o)
-        output = C.scatter_pairs_to_nodes(force_o, order, count, ctx.num_nodes)
+        output = C.electric_force_nodes(g, fx.view(-1), fy.view(-1), xy_o, order, rec4, ratio_o,
+                                        op.num_movable_nodes, op.num_filler_nodes, ctx.num_nodes, float(op.xl),
+                                        float(op.yl), float(op.bin_size_x), float(op.bin_size_y), op.num_bins_x,
+                                        op.num_bins_y, -1.0)
         return output, None, None, None, None
 
 
@@ -607,7 +616,5 @@ class ElectricPotential(ElectricOverflow):
         if mode == "density":
             return ElectricPotentialOrderedFunction.apply(pos, self, self.precision, self.fast_mode,
                                                           self.recompute_field)
-        density_map, _ = self.ordered_density_map(pos, 0)
-        bin_area = self.bin_size_x * self.bin_size_y
-        out = C.density_overflow(density_map, float(self.target_density * bin_area), float(bin_area))
-        return out[0].float(), out[1].float()
+        out = self.ordered_density_map(pos, 0, overflow=True)[2][1]
+        return out[0], out[1]

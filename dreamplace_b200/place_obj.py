@@ -15,6 +15,7 @@ import torch
 from torch import nn
 
 from . import electric_potential as ep_mod
+from ._native import C
 from .placement_ops import HPWL, MoveBoundary, PinPos, PinWeightSum
 from .weighted_average_wirelength import WeightedAverageWirelength
 
@@ -106,6 +107,12 @@ class PreconditionOp(object):
         with torch.no_grad():
             if self._pws is None:
                 self._pws = self.ops.pws_op(self.data.net_weights)
+            lam = density_weight
+            if isinstance(lam, torch.Tensor) and lam.numel() == 1 and grad.is_cuda and grad.is_contiguous() and \
+                    all(t.device == grad.device and t.dtype == torch.float32 for t in (grad, lam)):
+                C.precondition(grad, self._pws, self.data.node_areas, lam, float(self.alpha))
+                self.iteration += 1
+                return grad
             precond = self._pws + self.alpha * density_weight * self.data.node_areas
             precond.clamp_(min=1.0)
             n = self.design.num_nodes

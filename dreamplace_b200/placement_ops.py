@@ -74,7 +74,8 @@ class HPWL(nn.Module):
         return C.hpwl_forward(pos.view(-1), self.flat_netpin, self.netpin_start, self.net_weights, self.net_mask)
 
     def forward(self, pos):
-        return self.forward_f64(pos)[0].float()
+        require_cuda(pos, "pos")
+        return C.hpwl_forward_f32(pos.view(-1), self.flat_netpin, self.netpin_start, self.net_weights, self.net_mask)
 
 
 class MoveBoundary(object):

@@ -50,8 +50,15 @@ class WeightedAverageWirelengthLanesFunction(Function):
     dp_wa_pins_backward)."""
 
     @staticmethod
-    def forward(ctx, pos, lanes, net_weights, net_mask, pin_mask, inv_gamma):
+    def forward(ctx, pos, lanes, net_weights, net_mask, pin_mask, inv_gamma, gamma=None):
+        """gamma (a float32 CUDA scalar): given, inv_gamma is not read."""
         require_cuda(pos, "pos")
+        if gamma is not None:
+            grad_lane = torch.empty(2 * lanes.num_slots, dtype=torch.float32, device=pos.device)
+            value = C.wa_pins_value(pos.view(pos.numel()), lanes.group_deg, lanes.group_base, lanes.group_net,
+                                    lanes.ln_pin, net_weights, net_mask, gamma, grad_lane)
+            ctx.lanes, ctx.grad_lane, ctx.pin_mask = lanes, grad_lane, pin_mask
+            return value
         wl64 = torch.empty(REDUCE_DOUBLES, dtype=torch.float64, device=pos.device)
         grad_lane = torch.empty(2 * lanes.num_slots, dtype=torch.float32, device=pos.device)
         ig = inv_gamma.reshape(1).to(torch.float32)
@@ -67,7 +74,7 @@ class WeightedAverageWirelengthLanesFunction(Function):
         g = grad_pos.reshape(1).to(torch.float32)
         mask = ctx.pin_mask.view(torch.uint8) if ctx.pin_mask is not None else None
         output = C.wa_pins_backward(ctx.grad_lane, ctx.lanes.lane_of_pin, mask, g)
-        return output, None, None, None, None, None
+        return output, None, None, None, None, None, None
 
 
 class WeightedAverageWirelengthMergedFunction(Function):
@@ -123,5 +130,10 @@ class WeightedAverageWirelength(nn.Module):
         if self.lanes is None:
             require_cuda(pos, "pos")
             self.lanes = PinLanes(self.flat_netpin, self.netpin_start)
+        g = self.gamma
+        if isinstance(g, torch.Tensor) and g.is_cuda and g.device == pos.device and g.dtype == torch.float32 and \
+                g.numel() == 1 and not g.requires_grad and pos.dtype == torch.float32:
+            return WeightedAverageWirelengthLanesFunction.apply(pos, self.lanes, self.net_weights, self.net_mask,
+                                                                self.pin_mask, None, g)
         return WeightedAverageWirelengthLanesFunction.apply(pos, self.lanes, self.net_weights, self.net_mask,
                                                             self.pin_mask, 1.0 / self.gamma)

@@ -508,6 +508,37 @@ int dp_scatter_pairs_to_nodes(const float* vals_o, const int* order, int count, 
  * counterpart). */
 int dp_trial_metrics(const double* hpwl, const double* overflow2, const double* state, const double* obj,
                      const double* wl, const double* energy, double* out8, dp_stream_t stream);
+/* ---- the module path's calls in as few launches as they need ------------------
+ * The density map of the cells of a visiting order (dp_order_cells_by_bin; cells
+ * [0, num_first) and [num_first, count) each start a scatter block):
+ * out = (initial_density_map + cells) * scale, their positions in visiting
+ * order into xy_o, and optionally dp_density_overflow of the unscaled map. */
+int dp_density_cells(const float* pos, int num_nodes, const int* order, const float* rec4, const float* ratio_o,
+                     int num_first, int count, const float* initial_density_map, float xl, float yl, float xh,
+                     float yh, float bin_size_x, float bin_size_y, float inv_bin_size_x, float inv_bin_size_y,
+                     int num_bins_x, int num_bins_y, int deterministic, int fraction_bits, int64_t* scratch_fixed,
+                     float scale, float* xy_o, float* out, double target_area, double bin_area,
+                     double* overflow_f64, float* overflow_f32, dp_stream_t stream);
+/* dp_electric_force_ordered written in node order (out = [x(n) | y(n)], zero for
+ * the nodes between the movable cells and the fillers) */
+int dp_electric_force_nodes(const float* grad_pos, int num_bins_x, int num_bins_y, const float* field_map_x,
+                            const float* field_map_y, const float* xy_o, const int* order, const float* rec4,
+                            const float* ratio_o, int num_movable, int num_filler, int num_nodes, float xl, float yl,
+                            float bin_size_x, float bin_size_y, float inv_bin_size_x, float inv_bin_size_y,
+                            float scale, float* out, dp_stream_t stream);
+/* dp_pin_pos_forward through an interleaved copy of the positions (xy_work,
+ * 2 num_nodes floats, 8-byte aligned) */
+int dp_pin_pos_forward_xy(const float* pos, int num_nodes, const float* pin_offset_x, const float* pin_offset_y,
+                          const int* pin2node_map, int num_pins, float* xy_work, float* pin_pos, dp_stream_t stream);
+/* dp_wa_pins_forward given gamma (its reciprocal is taken in the kernel), the
+ * value also rounded to float */
+int dp_wa_pins_value(const float* pin_pos, int num_pins, const int* group_deg, const int* group_base,
+                     const int* group_net, int num_groups, const int* ln_pin, const float* net_weights,
+                     const unsigned char* net_mask, const float* gamma, double* wl_f64, float* grad_lane,
+                     float* wl_f32, dp_stream_t stream);
+/* grad /= max(1, pws + alpha lambda area), x and y (dreamplace/PlaceObj.py:69-103) */
+int dp_precondition(float* grad, const float* pws, const float* area, const float* lambda_, float alpha,
+                    int num_nodes, dp_stream_t stream);
 /* ---- one Nesterov trial in as few launches as it needs ------------------------
  * The kernels of dp_iteration_head, dp_nesterov_trial, dp_wa_lanes_forward,
  * dp_density_map_ordered_split, dp_prepare_operand, dp_electric_force_ordered,
