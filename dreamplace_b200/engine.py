@@ -23,6 +23,7 @@ re-organised for the GPU:
   loop runs while the GPU computes, and iteration k+1 is enqueued again only
   when k needed a retry or the host changed what k+1 reads.
 """
+import collections
 import math
 
 import numpy as np
@@ -40,6 +41,22 @@ NSLOT = 3
 M_HPWL, M_OVF, M_MAXD, M_ACCEPT, M_ALPHA, M_OBJ, M_WL, M_ENERGY = range(8)
 # pieces of one Nesterov trial, in launch order
 PIECES = ("nesterov_trial", "wa_forward", "density_scatter", "poisson_gemms", "field_gather", "assemble_precondition")
+
+
+# (pinned metrics rows, events) of engines that are gone: the last trial enqueued
+# ahead writes its row without the host allocator's knowledge, so the rows are
+# given back by a later engine's set-up, once the events are done
+_RETIRED = collections.deque()
+
+
+def _release_retired():
+    for _ in range(len(_RETIRED)):
+        try:
+            rows, events = _RETIRED.popleft()
+        except IndexError:  # another thread took it
+            return
+        if not all(e.query() for e in events):
+            _RETIRED.append((rows, events))
 
 
 class GPEngine(object):
@@ -131,6 +148,7 @@ class GPEngine(object):
         self.O = [torch.zeros(REDUCE_DOUBLES, **f64) for _ in range(NSLOT)]
         self.metrics = [torch.zeros(8, **f64) for _ in range(NSLOT)]
         self.metrics_host = [torch.zeros(8, dtype=torch.float64, pin_memory=True) for _ in range(NSLOT)]
+        _release_retired()
         self.metrics_dev = [C.host_pointer(t) for t in self.metrics_host]
         self.ready = [None] * NSLOT
         self.grad_scale = torch.zeros(1, dtype=torch.float32, device=dev)
@@ -259,6 +277,11 @@ class GPEngine(object):
         median = key[mid] - torch.arange(num_nets, device=ns.device) * span
         median = torch.where(deg > 0, median, torch.zeros_like(median))
         return torch.argsort(median, stable=True).to(torch.int32).cpu()
+
+    def __del__(self):
+        events = [e for e in getattr(self, "ready", ()) if e is not None]
+        if events and _RETIRED is not None:  # (None while the interpreter exits)
+            _RETIRED.append((self.metrics_host, events))
 
     # ---------------------------------------------------------------- pieces
     def _build_records(self):
