@@ -325,8 +325,9 @@ at::Tensor pin_pos_forward(at::Tensor pos, at::Tensor offx, at::Tensor offy, at:
   c10::cuda::CUDAGuard guard(pos.device());
   int num_pins = offx.numel();
   auto out = at::empty({2 * (int64_t)num_pins}, pos.options());
-  // the interleaved copy costs a pass over the nodes and a launch, and pays
-  // from about a million pins
+  // the interleaved copy costs a pass over the nodes and a launch: at 7.1M pins
+  // 10 + 43 us against 68 planar, at 1.7M 2.8 + 11.2 against 16.6; below a
+  // million the launch costs what the sectors save (0.17M pins: 3.5 planar)
   constexpr int kPackPins = 1 << 20;
   if (num_pins >= kPackPins && num_pins >= pos.numel() / 2) {
     auto xy = at::empty_like(pos);

@@ -137,8 +137,8 @@ __global__ void __launch_bounds__(256) electric_force_records_kernel(
     gx = fmul(fmul(fmul(gx, r), g), scale);
     gy = fmul(fmul(fmul(gy, r), g), scale);
     if (nodes.out) {
-      // scattered words, which L2 merges: a pass of its own that put the pairs
-      // back in node order took 34 us of the 3.1M cells' 73
+      // scattered words, which L2 merges: at 3.1M cells 60 us; with a pass of
+      // its own that put the pairs back in node order 39 + 34 us
       const int i = __ldg(nodes.order + idx);
       nodes.out[i] = gx;
       nodes.out[nodes.num_nodes + i] = gy;

@@ -25,6 +25,8 @@ solve, us, product -> fast transform: split_bf16 64^2 26 -> 9, 1024^2 68 -> 25,
 name the arithmetic of a product, and stay one.
 """
 
+import functools
+
 import numpy as np
 import torch
 from torch import nn
@@ -148,11 +150,16 @@ def fft_table(n, device):
     return _FFT_TABLES[key]
 
 
+@functools.lru_cache(maxsize=None)
+def _fft_sides(M, N):
+    return bool(C.fft_supported(M, N))
+
+
 def fft_serves(x, prec):
     """Whether the fast transforms take this map: fp32 or split_bf16, sides that
     are powers of two in 64 .. 4096, rows that a bulk copy can start on."""
-    return prec in (0, 3) and x.is_cuda and x.dtype == torch.float32 and x.dim() == 2 and x.is_contiguous() and \
-        C.fft_supported(x.size(0), x.size(1)) and x.data_ptr() % 16 == 0
+    return prec in (0, 3) and x.dim() == 2 and _fft_sides(*x.shape) and x.is_cuda and x.dtype == torch.float32 and \
+        x.is_contiguous() and x.data_ptr() % 16 == 0
 
 
 def transform_2d(x, left, right, alpha, prec, out=None):
@@ -197,10 +204,12 @@ class _Transform(nn.Module):
         M, N = x.size(-2), x.size(-1)
         if self.out is None or self.out.shape != (M, N) or self.out.device != x.device:
             self.out = torch.empty(M, N, dtype=torch.float32, device=x.device)
-        x = x.reshape(M, N).contiguous()
-        if fft_serves(x, self.precision):
-            C.transform_fft(_FFT_KINDS[self.kind], x, fft_table(M, x.device), fft_table(N, x.device), self.out)
-            return self.out
+        x = x.reshape(M, N)
+        if self.precision in (0, 3) and _fft_sides(M, N):
+            x = x.contiguous()
+            if fft_serves(x, self.precision):
+                C.transform_fft(_FFT_KINDS[self.kind], x, fft_table(M, x.device), fft_table(N, x.device), self.out)
+                return self.out
         cM, chM, shM = transform_matrices(M, self.precision, x.device)
         cN, chN, shN = transform_matrices(N, self.precision, x.device)
         left, right, alpha = {
