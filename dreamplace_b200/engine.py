@@ -43,9 +43,9 @@ M_HPWL, M_OVF, M_MAXD, M_ACCEPT, M_ALPHA, M_OBJ, M_WL, M_ENERGY = range(8)
 PIECES = ("nesterov_trial", "wa_forward", "density_scatter", "poisson_gemms", "field_gather", "assemble_precondition")
 
 
-# (pinned metrics rows, events) of engines that are gone: the last trial enqueued
-# ahead writes its row without the host allocator's knowledge, so the rows are
-# given back by a later engine's set-up, once the events are done
+# (pinned metrics rows, events) of engines that are gone: a trial writes its row
+# without the host allocator's knowledge, so the rows are given back by a later
+# engine's set-up, once the events behind the last trials (_record_ready) are done
 _RETIRED = collections.deque()
 
 
@@ -670,7 +670,10 @@ class GPEngine(object):
                 st.wait_stream(torch.cuda.current_stream())
                 with torch.cuda.stream(st):
                     saved = self.S[s].clone()
-                    self._body(s, head)
+                    try:
+                        self._body(s, head)
+                    finally:
+                        self._record_ready(s)  # the warm-up trial writes the host's row too
                     self.S[s].copy_(saved)
                 torch.cuda.current_stream().wait_stream(st)
             # captured on a side stream with capture_begin / capture_end (the
@@ -707,8 +710,17 @@ class GPEngine(object):
             self.kernels_launched += self.graph_kernels[(s, head)]
         else:
             before = C.launch_count()
-            self._body(s, head)
+            try:
+                self._body(s, head)
+            finally:
+                self._record_ready(s)
             self.kernels_launched += C.launch_count() - before
+            return
+        self._record_ready(s)
+
+    def _record_ready(self, s):
+        """Marks, on the current stream, the end of the trial enqueued from slot s:
+        what the host waits for, and what keeps the metrics rows (__del__)."""
         if self.ready[s] is None:
             self.ready[s] = torch.cuda.Event()
         self.ready[s].record(self._current_stream())

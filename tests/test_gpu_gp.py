@@ -302,3 +302,25 @@ def test_fused_trial_equals_its_pieces(design, precision, deterministic):
         # the energy is an atomic fp64 sum of the solve's tiles: its last bits vary
         rel = 1e-12 if deterministic and k in ("row", "host") else 0.0 if deterministic else 1e-4
         assert (got[k].double() - v.double()).abs().max() <= rel * v.double().abs().max(), k
+
+
+def test_pinned_rows_outlive_the_warm_up_of_the_graphs(design):
+    """A trial's last kernel writes the host's metrics row, which the pinned
+    allocator does not see.  The warm-up of the graphs enqueues such a trial
+    before any step has: an engine dropped then keeps its rows until that trial
+    is done, and the next engine's set-up gives them back."""
+    import gc
+    from dreamplace_b200 import engine
+    placer, _, _ = run(design, "graph", "fp32", 2, deterministic=1)
+    first = placer.stepper.eng
+    eng = engine.GPEngine(placer.params, design, placer.data_collections, placer.op_collections, placer.model, True)
+    eng.load_state_dict(first.state_dict())
+    eng._check_graph_key()
+    eng._graph(eng.slot, False)
+    rows = eng.metrics_host
+    del eng
+    gc.collect()
+    assert any(kept is rows for kept, _ in engine._RETIRED)
+    torch.cuda.synchronize()
+    engine._release_retired()
+    assert not any(kept is rows for kept, _ in engine._RETIRED)
