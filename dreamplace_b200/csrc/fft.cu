@@ -225,7 +225,9 @@ __device__ __forceinline__ float2 idct_pack(int k, float2 ak, float2 an, float2 
 // so each row is read once in full lines whatever order the permutation asks
 // for.  The wait for the copies is bounded like the tensor-core GEMM's
 // (dp_tc_set_wait_budget): on expiry status 2 is recorded (dp_tc_status) and
-// the block returns.
+// the block returns, once its copies have landed (a second wait, bounded by
+// kFftDrainCycles whatever the budget): a block that is gone must not have its
+// shared memory written.
 __device__ int g_fft_status = 0;
 __device__ long long g_fft_wait_budget = 4000000000ll;  // ~2 s at 2 GHz
 __device__ int g_fft_skip_loads = 0;                    // test hook (dp_tc_set_skip_loads)
@@ -252,6 +254,14 @@ __device__ __noinline__ bool fft_bounded_wait(uint64_t* bar) {
       return false;
     }
   return true;
+}
+
+constexpr long long kFftDrainCycles = 4000000000ll;  // ~2 s at 2 GHz
+
+__device__ __noinline__ void fft_drain(uint64_t* bar) {
+  const long long start = clock64();
+  while (!fft_try_wait(bar) && clock64() - start <= kFftDrainCycles) {
+  }
 }
 
 enum { kRowDct = 0, kRowInv = 1, kRowInvPairs = 2 };
@@ -296,13 +306,15 @@ __global__ void __launch_bounds__(RowBlock<LOGN>::kThreads) fft_rows_kernel(RowA
   const int f = threadIdx.x / S::T, t = threadIdx.x % S::T;
   const int first = blockIdx.x * B::F;
   const int here = min(B::F, a.count - first);
+  int skip = 0;
   if (threadIdx.x == 0) {
     if (a.zero && blockIdx.x == 0) *a.zero = 0.0;
+    skip = g_fft_skip_loads;
     constexpr uint32_t kBytes = 2 * S::N * sizeof(float);
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fft_smem_addr(&bar)),
                  "r"(kBytes * here)
                  : "memory");
-    for (int i = 0; i < here && !g_fft_skip_loads; ++i)
+    for (int i = 0; i < here && !skip; ++i)
       asm volatile(
           "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
               fft_smem_addr(fft_smem + i * S::PITCH)),
@@ -310,7 +322,10 @@ __global__ void __launch_bounds__(RowBlock<LOGN>::kThreads) fft_rows_kernel(RowA
           : "memory");
   }
   __syncthreads();
-  if (!__syncthreads_and(fft_try_wait(&bar) || fft_bounded_wait(&bar))) return;
+  if (!__syncthreads_and(fft_try_wait(&bar) || fft_bounded_wait(&bar))) {
+    if (threadIdx.x == 0 && !skip) fft_drain(&bar);  // the block lives until its last thread returns
+    return;
+  }
   float2* s = fft_smem + f * S::PITCH;
   const float2* W = a.tw + S::N;
   const bool live = f < here;  // every thread takes part in the barriers

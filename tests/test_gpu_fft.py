@@ -110,3 +110,25 @@ def test_product_bounded_wait_on_a_ragged_grid(C):
     assert status == 2
     assert torch.equal(poisson_solve(x, 10.0, 10.0, "split_bf16")[0], before)
     assert C.tc_status() == 0
+
+
+def test_row_wait_that_expires_with_its_copies_in_flight(C):
+    """A wait budget shorter than the copies take: blocks that give up wait for
+    what they issued before they return, the status says so, and the next solve
+    is what it was."""
+    from dreamplace_b200.electric_potential import poisson_solve
+    for side in (64, 1024, 4096):
+        x = torch.from_numpy(density(side, side, 7)).cuda()
+        before = [t.clone() for t in poisson_solve(x, 10.0, 10.0, "fp32")]
+        assert C.tc_status() == 0
+        try:
+            C.tc_set_wait_budget(1)
+            for _ in range(3):
+                poisson_solve(x, 10.0, 10.0, "fp32")
+            status = C.tc_status()
+        finally:
+            C.tc_set_wait_budget(4_000_000_000)
+        assert status in (0, 2)  # the hardware's own wait may outlast the copies
+        after = poisson_solve(x, 10.0, 10.0, "fp32")
+        assert torch.equal(after[0], before[0]) and torch.equal(after[1], before[1])
+        assert C.tc_status() == 0
