@@ -2,8 +2,8 @@
 //
 // Each function checks its tensors the way the reference's pybind ops do
 // (CHECK_FLAT_CUDA / CHECK_CONTIGUOUS / CHECK_EVEN, utility/src/torch.h:62-76),
-// allocates outputs through the caching allocator, launches on the current
-// stream and turns a non-zero C ABI status into a Python RuntimeError.
+// allocates outputs through the caching allocator, launches on the current stream
+// of its tensors' device and turns a non-zero C ABI status into a Python RuntimeError.
 // Function names and argument order follow the reference ops they replace:
 //   electric_potential_cuda.{density_map, fixed_density_map, electric_force}
 //   weighted_average_wirelength_cuda_merged.{forward, backward}
@@ -182,8 +182,10 @@ static T dict_get(const py::dict& d, const char* key, T dflt) {
 
 void transform_gemm(int precision, int M, int N, int K, py::list problems) {
   std::vector<dp_gemm_problem> probs;
+  c10::cuda::OptionalCUDAGuard guard;
   for (auto item : problems) {
     py::dict d = item.cast<py::dict>();
+    if (probs.empty() && tensor_ptr(d, "a_hi")) guard.set_device(d["a_hi"].cast<at::Tensor>().device());
     dp_gemm_problem q;
     memset(&q, 0, sizeof(q));
     q.a_hi = tensor_ptr(d, "a_hi"); q.a_lo = tensor_ptr(d, "a_lo");
@@ -214,12 +216,15 @@ void transform_gemm(int precision, int M, int N, int K, py::list problems) {
 void prepare_operand(int precision, at::Tensor x, double scale, c10::optional<at::Tensor> out_f32,
                      c10::optional<at::Tensor> out_hi, c10::optional<at::Tensor> out_lo) {
   CHECK_CUDA_T(x); CHECK_CONTIG(x); CHECK_F32(x);
+  c10::cuda::CUDAGuard guard(x.device());
   DP_CALL(dp_prepare_operand(precision, ptr<float>(x), x.numel(), (float)scale, optr<float>(out_f32),
                              out_hi.has_value() ? out_hi->data_ptr() : nullptr,
                              out_lo.has_value() ? out_lo->data_ptr() : nullptr, cur_stream()));
 }
 
 at::Tensor spectral_weights(int M, int N, double wv_scale, at::Device device) {
+  c10::cuda::OptionalCUDAGuard guard;
+  if (device.has_index()) guard.set_device(device);
   auto out = at::empty({3, M, N}, at::TensorOptions().dtype(at::kFloat).device(device));
   DP_CALL(dp_spectral_weights(M, N, (float)wv_scale, ptr<float>(out), cur_stream()));
   return out;
@@ -402,13 +407,17 @@ static void* ovp(const c10::optional<at::Tensor>& t) {
   return (t.has_value() && t->defined() && t->numel() > 0) ? t->data_ptr() : nullptr;
 }
 
-void nesterov_init(at::Tensor state, double alpha) { DP_CALL(dp_nesterov_init(ptr<double>(state), alpha, cur_stream())); }
+void nesterov_init(at::Tensor state, double alpha) {
+  c10::cuda::CUDAGuard guard(state.device());
+  DP_CALL(dp_nesterov_init(ptr<double>(state), alpha, cur_stream()));
+}
 
 void nesterov_trial(at::Tensor v, at::Tensor g, at::Tensor u, at::Tensor u_new, at::Tensor v_new,
                     c10::optional<at::Tensor> xy_new, at::Tensor state, at::Tensor sx, at::Tensor sy, double xl,
                     double yl, double xh, double yh, int num_movable, int num_filler,
                     c10::optional<at::Tensor> inv_order, c10::optional<at::Tensor> xy_order) {
   TORCH_CHECK(!xy_order.has_value() || inv_order.has_value(), "xy_order needs inv_order");
+  c10::cuda::CUDAGuard guard(v.device());
   DP_CALL(dp_nesterov_trial(ptr<float>(v), ptr<float>(g), ptr<float>(u), ptr<float>(u_new), ptr<float>(v_new),
                             (float*)ovp(xy_new), ptr<double>(state), ptr<float>(sx), ptr<float>(sy), xl, yl, xh, yh,
                             v.numel() / 2, num_movable, num_filler, (const int*)ovp(inv_order),
@@ -418,17 +427,20 @@ void nesterov_trial(at::Tensor v, at::Tensor g, at::Tensor u, at::Tensor u_new, 
 void gather_order_xy(at::Tensor xy, at::Tensor order, int count, at::Tensor xy_o) {
   CHECK_FLAT(xy); CHECK_F32(xy); CHECK_I32(order); CHECK_F32(xy_o);
   TORCH_CHECK(count <= order.numel() && 2 * count <= xy_o.numel(), "gather_order_xy: buffers smaller than count");
+  c10::cuda::CUDAGuard guard(xy.device());
   DP_CALL(dp_gather_order_xy(ptr<float>(xy), ptr<int>(order), count, ptr<float>(xy_o), cur_stream()));
 }
 
 void pack_xy(at::Tensor pos, at::Tensor xy) {
   CHECK_F32(pos); CHECK_F32(xy);
   TORCH_CHECK(xy.numel() == pos.numel(), "xy must have as many elements as pos");
+  c10::cuda::CUDAGuard guard(pos.device());
   DP_CALL(dp_pack_xy(ptr<float>(pos), pos.numel() / 2, ptr<float>(xy), cur_stream()));
 }
 
 void precondition_step_size(at::Tensor g_new, at::Tensor g, at::Tensor v_new, at::Tensor v, at::Tensor pws,
                             at::Tensor area, at::Tensor lam, at::Tensor state) {
+  c10::cuda::CUDAGuard guard(g_new.device());
   DP_CALL(dp_precondition_step_size(ptr<float>(g_new), ptr<float>(g), ptr<float>(v_new), ptr<float>(v),
                                     ptr<float>(pws), ptr<float>(area), ptr<float>(lam), g_new.numel() / 2,
                                     ptr<double>(state), cur_stream()));
@@ -447,6 +459,7 @@ void iteration_head(at::Tensor state_prev, at::Tensor state_new, at::Tensor sche
                   weights_new.numel() >= 3,
               "iteration_head: buffers too small");
   CHECK_F32(weights_prev); CHECK_F32(weights_new);
+  c10::cuda::CUDAGuard guard(state_prev.device());
   DP_CALL(dp_iteration_head(ptr<double>(state_prev), ptr<double>(state_new), ptr<double>(sched_prev),
                             ptr<double>(sched_new), ptr<double>(hpwl_k), ptr<double>(overflow_k),
                             ptr<float>(weights_prev), ptr<float>(weights_new), base_gamma, total_area, ref_hpwl,
@@ -464,6 +477,7 @@ void set_trial_gate(c10::optional<at::Tensor> gate) {
 
 void trial_gate(at::Tensor gate, c10::optional<at::Tensor> accept_prev) {
   CHECK_I32(gate);
+  c10::cuda::CUDAGuard guard(gate.device());
   DP_CALL(dp_trial_gate(ptr<int>(gate), accept_prev.has_value() ? ptr<double>(*accept_prev) : nullptr,
                         cur_stream()));
 }
@@ -472,6 +486,7 @@ void objective_finish(c10::optional<at::Tensor> wl, at::Tensor energy, at::Tenso
                       at::Tensor factor_quad, c10::optional<at::Tensor> obj, c10::optional<at::Tensor> grad_scale) {
   CHECK_F32(factor_quad);
   TORCH_CHECK(factor_quad.numel() >= 2, "factor_quad holds (density_factor, quad_c)");
+  c10::cuda::CUDAGuard guard(energy.device());
   DP_CALL(dp_objective_finish(wl.has_value() ? ptr<double>(*wl) : nullptr, ptr<double>(energy),
                               ptr<float>(density_weight), ptr<float>(factor_quad),
                               obj.has_value() ? ptr<double>(*obj) : nullptr,
@@ -484,6 +499,7 @@ void build_cell_records(at::Tensor sx, at::Tensor sy, at::Tensor ox, at::Tensor 
   CHECK_I32(order); CHECK_F32(rec4); CHECK_F32(ratio_o);
   TORCH_CHECK(count <= order.numel() && 4 * count <= rec4.numel() && count <= ratio_o.numel(),
               "build_cell_records: buffers smaller than count");
+  c10::cuda::CUDAGuard guard(sx.device());
   DP_CALL(dp_build_cell_records(ptr<float>(sx), ptr<float>(sy), ptr<float>(ox), ptr<float>(oy), ptr<float>(ratio),
                                 ptr<int>(order), count, ptr<float>(rec4), ptr<float>(ratio_o), (int*)ovp(inv_order),
                                 cur_stream()));
@@ -502,6 +518,7 @@ void density_map_ordered_into(at::Tensor xy_o, at::Tensor rec4, at::Tensor ratio
               "density_map_ordered_into: buffers smaller than count");
   TORCH_CHECK(out.numel() == (int64_t)nbx * nby, "density_map_ordered_into: output is not num_bins_x*num_bins_y");
   TORCH_CHECK(!deterministic || scratch.has_value(), "deterministic mode needs the int64 scratch map");
+  c10::cuda::CUDAGuard guard(xy_o.device());
   DP_CALL(dp_density_map_ordered(ptr<float>(xy_o), (const int*)ovp(order), ptr<float>(rec4), ptr<float>(ratio_o),
                                  count,
                                  (const float*)ovp(init), xl, yl, xh, yh, bsx, bsy, inv_f(bsx), inv_f(bsy), nbx, nby,
@@ -528,6 +545,7 @@ void density_map_ordered_split(at::Tensor xy_o, at::Tensor rec4, at::Tensor rati
   TORCH_CHECK(out_first.numel() == (int64_t)nbx * nby && out_all.numel() == out_first.numel(),
               "density_map_ordered_split: outputs are not num_bins_x*num_bins_y");
   TORCH_CHECK(!deterministic || scratch.has_value(), "deterministic mode needs the int64 scratch map");
+  c10::cuda::CUDAGuard guard(xy_o.device());
   DP_CALL(dp_density_map_ordered_split(ptr<float>(xy_o), (const int*)ovp(order), ptr<float>(rec4),
                                        ptr<float>(ratio_o),
                                        num_first, count, (const float*)ovp(init), xl, yl, xh, yh, bsx, bsy,
@@ -547,6 +565,7 @@ void electric_force_ordered(at::Tensor grad_scale, at::Tensor ex, at::Tensor ey,
   TORCH_CHECK(2 * count <= xy_o.numel() && 4 * count <= rec4.numel() && 2 * count <= force_o.numel(),
               "electric_force_ordered: buffers smaller than count");
   TORCH_CHECK(ex.numel() == (int64_t)nbx * nby && ey.numel() == ex.numel(), "electric_force_ordered: field map size");
+  c10::cuda::CUDAGuard guard(grad_scale.device());
   DP_CALL(dp_electric_force_ordered(ptr<float>(grad_scale), nbx, nby, ptr<float>(ex), ptr<float>(ey), ptr<float>(xy_o),
                                     (const int*)ovp(order),
                                     ptr<float>(rec4), ptr<float>(ratio_o), count, xl, yl, bsx, bsy,
@@ -561,6 +580,7 @@ void assemble_precondition_step(at::Tensor grad_node_order, at::Tensor node_star
   int n = v.numel() / 2;
   TORCH_CHECK(inv_order.numel() >= n && node_start.numel() >= num_movable + 1 && g_new.numel() == 2 * n,
               "assemble_precondition_step: size mismatch");
+  c10::cuda::CUDAGuard guard(grad_node_order.device());
   DP_CALL(dp_assemble_precondition_step(ptr<float>(grad_node_order), ptr<int>(node_start), ptr<float>(wl_scale),
                                         ptr<float>(force_o), ptr<int>(inv_order), num_movable, num_filler,
                                         ptr<float>(pws), ptr<float>(area), ptr<float>(lambda_), n, ptr<float>(v_new),
@@ -569,6 +589,7 @@ void assemble_precondition_step(at::Tensor grad_node_order, at::Tensor node_star
 }
 
 void density_overflow_into(at::Tensor density_map, double target_area, double bin_area, at::Tensor out2) {
+  c10::cuda::CUDAGuard guard(density_map.device());
   DP_CALL(dp_density_overflow(ptr<float>(density_map), density_map.numel(), target_area, bin_area, ptr<double>(out2),
                               nullptr, cur_stream()));
 }
@@ -577,6 +598,7 @@ void electric_force_into(at::Tensor grad_scale, at::Tensor ex, at::Tensor ey, at
                          at::Tensor sy, at::Tensor ox, at::Tensor oy, at::Tensor ratio, double xl, double yl,
                          double xh, double yh, double bsx, double bsy, int nbx, int nby, int num_movable,
                          int num_filler, c10::optional<at::Tensor> sorted_node_map, double scale, at::Tensor out) {
+  c10::cuda::CUDAGuard guard(grad_scale.device());
   DP_CALL(dp_electric_force(ptr<float>(grad_scale), nbx, nby, ptr<float>(ex), ptr<float>(ey), ptr<float>(pos),
                             pos.numel() / 2, ptr<float>(sx), ptr<float>(sy), ptr<float>(ox), ptr<float>(oy),
                             ptr<float>(ratio), xl, yl, xh, yh, bsx, bsy, inv_f(bsx), inv_f(bsy), num_movable,
@@ -618,6 +640,7 @@ void wa_lanes_forward(at::Tensor xy, at::Tensor group_deg, at::Tensor group_base
   TORCH_CHECK(!hpwl_f64.has_value() || (hpwl_mask.has_value() && hpwl_f64->scalar_type() == at::kDouble &&
                                         hpwl_f64->numel() >= DP_REDUCE_DOUBLES),
               "hpwl_f64 needs hpwl_mask and DP_REDUCE_DOUBLES doubles");
+  c10::cuda::CUDAGuard guard(xy.device());
   DP_CALL(dp_wa_lanes_forward(ptr<float>(xy), ptr<int>(group_deg), ptr<int>(group_base), ptr<int>(group_net),
                               group_deg.numel(), ptr<int>(ln_node), ptr<float>(ln_offx), ptr<float>(ln_offy),
                               (const int*)ovp(ln_csr), (const float*)ovp(net_weights), net_mask.data_ptr<uint8_t>(),
@@ -632,6 +655,7 @@ void hpwl_lanes(at::Tensor xy, at::Tensor group_deg, at::Tensor group_base, at::
   CHECK_FLAT(xy); CHECK_I32(group_deg); CHECK_I32(group_base); CHECK_I32(group_net); CHECK_I32(ln_node);
   TORCH_CHECK(group_net.numel() == 32 * group_deg.numel(), "hpwl_lanes: inconsistent plan");
   TORCH_CHECK(out_f64.scalar_type() == at::kDouble && out_f64.numel() >= DP_REDUCE_DOUBLES, "out_f64 too small");
+  c10::cuda::CUDAGuard guard(xy.device());
   DP_CALL(dp_hpwl_lanes(ptr<float>(xy), ptr<int>(group_deg), ptr<int>(group_base), ptr<int>(group_net),
                         group_deg.numel(), ptr<int>(ln_node), ptr<float>(ln_offx), ptr<float>(ln_offy),
                         (const float*)ovp(net_weights), net_mask.data_ptr<uint8_t>(), ptr<double>(out_f64),
@@ -641,6 +665,7 @@ void hpwl_lanes(at::Tensor xy, at::Tensor group_deg, at::Tensor group_base, at::
 void node_pin_sum(at::Tensor grad_node_order, at::Tensor node_start, at::Tensor grad_pos, int num_movable,
                   int accumulate, at::Tensor grad_out) {
   CHECK_F32(grad_node_order); CHECK_F32(grad_out); CHECK_I32(node_start);
+  c10::cuda::CUDAGuard guard(grad_node_order.device());
   DP_CALL(dp_node_pin_sum(ptr<float>(grad_node_order), grad_node_order.numel() / 2, ptr<int>(node_start),
                           ptr<float>(grad_pos), num_movable, grad_out.numel() / 2, accumulate, ptr<float>(grad_out),
                           cur_stream()));
@@ -655,6 +680,7 @@ void wa_pins_forward(at::Tensor pin_pos, at::Tensor group_deg, at::Tensor group_
               "wa_pins_forward: inconsistent plan");
   TORCH_CHECK(grad_lane.numel() >= 2 * ln_pin.numel(), "wa_pins_forward: grad_lane smaller than the lane slots");
   TORCH_CHECK(wl_f64.scalar_type() == at::kDouble && wl_f64.numel() >= DP_REDUCE_DOUBLES, "wl_f64 too small");
+  c10::cuda::CUDAGuard guard(pin_pos.device());
   DP_CALL(dp_wa_pins_forward(ptr<float>(pin_pos), pin_pos.numel() / 2, ptr<int>(group_deg), ptr<int>(group_base),
                              ptr<int>(group_net), group_deg.numel(), ptr<int>(ln_pin), (const float*)ovp(net_weights),
                              net_mask.data_ptr<uint8_t>(), ptr<float>(inv_gamma), ptr<double>(wl_f64),
@@ -671,6 +697,7 @@ at::Tensor wa_pins_value(at::Tensor pin_pos, at::Tensor group_deg, at::Tensor gr
               "wa_pins_value: inconsistent plan");
   TORCH_CHECK(grad_lane.numel() >= 2 * ln_pin.numel(), "wa_pins_value: grad_lane smaller than the lane slots");
   TORCH_CHECK(gamma.numel() == 1, "wa_pins_value: gamma must hold one value");
+  c10::cuda::CUDAGuard guard(pin_pos.device());
   auto buf = at::empty({DP_REDUCE_DOUBLES}, pin_pos.options().dtype(at::kDouble));
   auto out = at::empty({}, pin_pos.options());
   DP_CALL(dp_wa_pins_value(ptr<float>(pin_pos), pin_pos.numel() / 2, ptr<int>(group_deg), ptr<int>(group_base),
@@ -722,6 +749,7 @@ at::Tensor electric_force_nodes(at::Tensor grad_pos, at::Tensor ex, at::Tensor e
                   count <= order.numel(),
               "electric_force_nodes: buffers smaller than the cells");
   TORCH_CHECK(ex.numel() == (int64_t)nbx * nby && ey.numel() == ex.numel(), "electric_force_nodes: field map size");
+  c10::cuda::CUDAGuard guard(grad_pos.device());
   auto out = at::empty({2 * (int64_t)num_nodes}, xy_o.options());
   DP_CALL(dp_electric_force_nodes(ptr<float>(grad_pos), nbx, nby, ptr<float>(ex), ptr<float>(ey), ptr<float>(xy_o),
                                   ptr<int>(order), ptr<float>(rec4), ptr<float>(ratio_o), num_movable, num_filler,
@@ -735,6 +763,7 @@ void precondition(at::Tensor grad, at::Tensor pws, at::Tensor area, at::Tensor l
   CHECK_CUDA_T(lam); CHECK_CONTIG(pws); CHECK_CONTIG(area);
   const int64_t n = grad.numel() / 2;
   TORCH_CHECK(pws.numel() == n && area.numel() == n && lam.numel() == 1, "precondition: size mismatch");
+  c10::cuda::CUDAGuard guard(grad.device());
   DP_CALL(dp_precondition(ptr<float>(grad), ptr<float>(pws), ptr<float>(area), ptr<float>(lam), (float)alpha, (int)n,
                           cur_stream()));
 }
@@ -745,6 +774,7 @@ at::Tensor wa_pins_backward(at::Tensor grad_lane, at::Tensor lane_of_pin, c10::o
   const int64_t P = lane_of_pin.numel();
   TORCH_CHECK(!pin_mask.has_value() || (pin_mask->numel() == P && pin_mask->element_size() == 1),
               "wa_pins_backward: pin_mask must hold one byte per pin");
+  c10::cuda::CUDAGuard guard(grad_lane.device());
   auto out = at::empty({2 * P}, grad_lane.options());
   DP_CALL(dp_wa_pins_backward(ptr<float>(grad_lane), ptr<int>(lane_of_pin),
                               pin_mask.has_value() ? (const unsigned char*)pin_mask->data_ptr() : nullptr,
@@ -760,6 +790,7 @@ void order_cells_by_bin(at::Tensor pos, at::Tensor ox, at::Tensor oy, int num_mo
                         double yl, double bsx, double bsy, int nbx, int nby, at::Tensor scratch, at::Tensor order) {
   CHECK_FLAT(pos); CHECK_F32(pos); CHECK_EVEN(pos); CHECK_I32(order); CHECK_CUDA_T(scratch); CHECK_CONTIG(scratch);
   TORCH_CHECK(order.numel() >= num_movable + num_filler, "order_cells_by_bin: order too small");
+  c10::cuda::CUDAGuard guard(pos.device());
   DP_CALL(dp_order_cells_by_bin(ptr<float>(pos), pos.numel() / 2, ptr<float>(ox), ptr<float>(oy), num_movable,
                                 num_filler, xl, yl, inv_f(bsx), inv_f(bsy), nbx, nby, scratch.data_ptr(),
                                 (size_t)scratch.numel() * scratch.element_size(), ptr<int>(order), cur_stream()));
@@ -768,6 +799,7 @@ void order_cells_by_bin(at::Tensor pos, at::Tensor ox, at::Tensor oy, int num_mo
 void gather_order_pos(at::Tensor pos, at::Tensor order, int count, at::Tensor xy_o) {
   CHECK_FLAT(pos); CHECK_F32(pos); CHECK_I32(order); CHECK_F32(xy_o);
   TORCH_CHECK(order.numel() >= count && xy_o.numel() >= 2 * count, "gather_order_pos: buffers smaller than count");
+  c10::cuda::CUDAGuard guard(pos.device());
   DP_CALL(dp_gather_order_pos(ptr<float>(pos), pos.numel() / 2, ptr<int>(order), count, ptr<float>(xy_o),
                               cur_stream()));
 }
@@ -775,6 +807,7 @@ void gather_order_pos(at::Tensor pos, at::Tensor order, int count, at::Tensor xy
 at::Tensor scatter_pairs_to_nodes(at::Tensor vals_o, at::Tensor order, int count, int num_nodes) {
   CHECK_F32(vals_o); CHECK_I32(order);
   TORCH_CHECK(order.numel() >= count && vals_o.numel() >= 2 * count, "scatter_pairs_to_nodes: buffers too small");
+  c10::cuda::CUDAGuard guard(vals_o.device());
   auto out = at::empty({2 * (int64_t)num_nodes}, vals_o.options());
   DP_CALL(dp_scatter_pairs_to_nodes(ptr<float>(vals_o), ptr<int>(order), count, num_nodes, ptr<float>(out),
                                     cur_stream()));
@@ -824,6 +857,7 @@ void trial_start(c10::optional<std::vector<at::Tensor>> head, std::vector<double
     z[i] = zero[i].data_ptr();
     zb[i] = zero[i].nbytes();
   }
+  c10::cuda::CUDAGuard guard(v.device());
   DP_CALL(dp_trial_start(hd[0], hd[1], const_cast<double*>(hd[2]), hd[3], hd[4], w[0], const_cast<float*>(w[1]),
                          head_scalars[0], head_scalars[1], head_scalars[2], head_scalars[3], head_scalars[4],
                          gate.has_value() ? ptr<int>(*gate) : nullptr, ptr<float>(v), ptr<float>(g), ptr<float>(u),
@@ -842,6 +876,7 @@ int trial_wirelength(at::Tensor xy, at::Tensor group_deg, at::Tensor group_base,
   TORCH_CHECK(group_net.numel() == 32 * group_deg.numel() && group_base.numel() == group_deg.numel(),
               "trial_wirelength: inconsistent plan");
   int blocks = 0;
+  c10::cuda::CUDAGuard guard(xy.device());
   DP_CALL(dp_trial_wirelength(ptr<float>(xy), ptr<int>(group_deg), ptr<int>(group_base), ptr<int>(group_net),
                               group_deg.numel(), ptr<int>(ln_node), ptr<float>(ln_offx), ptr<float>(ln_offy),
                               (const int*)ovp(ln_csr), (const float*)ovp(net_weights), net_mask.data_ptr<uint8_t>(),
@@ -874,6 +909,7 @@ int trial_density(at::Tensor xy_o, c10::optional<at::Tensor> order, at::Tensor r
                                       all_lo->numel() == nbins),
               "trial_density: the split operand is two bfloat16 maps");
   int blocks = 0;
+  c10::cuda::CUDAGuard guard(xy_o.device());
   DP_CALL(dp_trial_density(ptr<float>(xy_o), (const int*)ovp(order), ptr<float>(rec4), ptr<float>(ratio_o), num_first,
                            count, (const float*)ovp(init), xl, yl, xh, yh, bsx, bsy, inv_f(bsx), inv_f(bsy), nbx, nby,
                            deterministic, fraction_bits(xl, yl, xh, yh), (int64_t*)ovp(scratch2),
@@ -891,6 +927,7 @@ void trial_force(at::Tensor energy, at::Tensor density_weight, at::Tensor factor
                   factor_quad.numel() >= 2,
               "trial_force: buffers smaller than count");
   TORCH_CHECK(ex.numel() == (int64_t)nbx * nby && ey.numel() == ex.numel(), "trial_force: field map size");
+  c10::cuda::CUDAGuard guard(energy.device());
   DP_CALL(dp_trial_force(dptr(energy, 1), ptr<float>(density_weight), ptr<float>(factor_quad), nbx, nby,
                          ptr<float>(ex), ptr<float>(ey), ptr<float>(xy_o), (const int*)ovp(order), ptr<float>(rec4),
                          ptr<float>(ratio_o), count, xl, yl, bsx, bsy, inv_f(bsx), inv_f(bsy), (float)scale,
@@ -905,6 +942,7 @@ int trial_assemble(at::Tensor grad_node_order, at::Tensor node_start, at::Tensor
   int n = v.numel() / 2, blocks = 0;
   TORCH_CHECK(inv_order.numel() >= n && node_start.numel() >= num_movable + 1 && g_new.numel() == 2 * n,
               "trial_assemble: size mismatch");
+  c10::cuda::CUDAGuard guard(grad_node_order.device());
   DP_CALL(dp_trial_assemble(ptr<float>(grad_node_order), ptr<int>(node_start), ptr<float>(wl_scale),
                             ptr<float>(force_o), ptr<int>(inv_order), num_movable, num_filler, ptr<float>(pws),
                             ptr<float>(area), ptr<float>(lambda_), n, ptr<float>(v_new), ptr<float>(v),
@@ -919,6 +957,7 @@ void trial_finish(at::Tensor wl, at::Tensor hpwl, int wa_blocks, at::Tensor over
                   double bin_area, at::Tensor energy, at::Tensor density_weight, at::Tensor factor_quad,
                   at::Tensor state, int norm_blocks, at::Tensor hpwl_v, at::Tensor overflow_v, at::Tensor obj,
                   at::Tensor out8, int64_t out8_host) {
+  c10::cuda::CUDAGuard guard(wl.device());
   DP_CALL(dp_trial_finish(dptr(wl, DP_REDUCE_DOUBLES), dptr(hpwl, DP_REDUCE_DOUBLES), wa_blocks,
                           dptr(overflow, DP_REDUCE_DOUBLES), overflow_blocks, bin_area, dptr(energy, 1),
                           ptr<float>(density_weight), ptr<float>(factor_quad),
@@ -975,11 +1014,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("trial_metrics", [](at::Tensor hpwl, at::Tensor overflow2, at::Tensor state, at::Tensor obj, at::Tensor wl,
                             at::Tensor energy, at::Tensor out8) {
     TORCH_CHECK(out8.scalar_type() == at::kDouble && out8.numel() >= 8, "trial_metrics: out8 needs 8 doubles");
+    c10::cuda::CUDAGuard guard(out8.device());
     DP_CALL(dp_trial_metrics(ptr<double>(hpwl), ptr<double>(overflow2), ptr<double>(state), ptr<double>(obj),
                              ptr<double>(wl), ptr<double>(energy), ptr<double>(out8), cur_stream()));
   });
   m.def("zero_", [](at::Tensor t) {
     CHECK_CUDA_T(t); CHECK_CONTIG(t);
+    c10::cuda::CUDAGuard guard(t.device());
     DP_CALL(dp_zero(t.data_ptr(), (size_t)t.numel() * t.element_size(), cur_stream()));
   });
   m.def("tc_set_wait_budget", [](long long cycles) { DP_CALL(dp_tc_set_wait_budget(cycles)); });

@@ -58,3 +58,18 @@ def test_extension_imports():
     assert precision_code("split_bf16") == 3
     with pytest.raises(ValueError):
         precision_code("fp8")
+
+
+def test_every_binding_that_launches_switches_to_its_tensors_device():
+    """cur_stream() is a stream of the current device: a function that launches on
+    it first makes its tensors' device the current one (a CUDAGuard), as torch's
+    own operators do, so that a model on another device keeps working."""
+    text = open(os.path.join(ROOT, "dreamplace_b200", "csrc", "binding.cpp")).read()
+    calls = [m.start() for m in re.finditer(r"cur_stream\(\)\)", text)]
+    assert len(calls) > 50
+    bad = []
+    for at in calls:  # its function's text so far: functions end at a brace in column 0, bound lambdas start at m.def
+        body = re.split(r"\n}\n|\n  m\.def\(", text[:at])[-1]
+        if "CUDAGuard guard" not in body:
+            bad.append(text[:at].count("\n") + 1)
+    assert not bad, "lines of binding.cpp that launch without a device guard: %s" % bad
