@@ -758,14 +758,20 @@ at::Tensor electric_force_nodes(at::Tensor grad_pos, at::Tensor ex, at::Tensor e
   return out;
 }
 
-void precondition(at::Tensor grad, at::Tensor pws, at::Tensor area, at::Tensor lam, double alpha) {
-  CHECK_CUDA_T(grad); CHECK_CONTIG(grad); CHECK_F32(grad); CHECK_F32(pws); CHECK_F32(area); CHECK_F32(lam);
-  CHECK_CUDA_T(lam); CHECK_CONTIG(pws); CHECK_CONTIG(area);
+// false, and nothing done, for operands the kernel has no form for: other than
+// contiguous float32 on one CUDA device, a lambda of more than one element
+bool precondition(at::Tensor grad, at::Tensor pws, at::Tensor area, at::Tensor lam, double alpha) {
   const int64_t n = grad.numel() / 2;
-  TORCH_CHECK(pws.numel() == n && area.numel() == n && lam.numel() == 1, "precondition: size mismatch");
+  if (!grad.is_cuda() || grad.numel() != 2 * n || pws.numel() != n || area.numel() != n || lam.numel() != 1)
+    return false;
+  for (auto* t : {&grad, &pws, &area, &lam})
+    if (t->device() != grad.device() || t->scalar_type() != at::kFloat || !t->is_contiguous()) return false;
   c10::cuda::CUDAGuard guard(grad.device());
   DP_CALL(dp_precondition(ptr<float>(grad), ptr<float>(pws), ptr<float>(area), ptr<float>(lam), (float)alpha, (int)n,
                           cur_stream()));
+  // grad has changed in place: autograd's check of saved tensors is to see it
+  if (!grad.is_inference()) grad.unsafeGetTensorImpl()->bump_version();
+  return true;
 }
 
 at::Tensor wa_pins_backward(at::Tensor grad_lane, at::Tensor lane_of_pin, c10::optional<at::Tensor> pin_mask,

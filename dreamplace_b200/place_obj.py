@@ -107,15 +107,15 @@ class PreconditionOp(object):
         with torch.no_grad():
             if self._pws is None:
                 self._pws = self.ops.pws_op(self.data.net_weights)
-            lam = density_weight
-            if isinstance(lam, torch.Tensor) and lam.numel() == 1 and grad.is_cuda and grad.is_contiguous() and \
-                    all(t.device == grad.device and t.dtype == torch.float32 for t in (grad, lam)):
-                C.precondition(grad, self._pws, self.data.node_areas, lam, float(self.alpha))
+            n = self.design.num_nodes
+            # one kernel, where it takes the operands' form
+            if isinstance(density_weight, torch.Tensor) and isinstance(self.alpha, (int, float)) and \
+                    grad.numel() == 2 * n and \
+                    C.precondition(grad, self._pws, self.data.node_areas, density_weight, float(self.alpha)):
                 self.iteration += 1
                 return grad
             precond = self._pws + self.alpha * density_weight * self.data.node_areas
             precond.clamp_(min=1.0)
-            n = self.design.num_nodes
             grad.view(2, n).div_(precond)
             self.iteration += 1
         return grad

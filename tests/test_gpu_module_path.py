@@ -95,7 +95,7 @@ def test_wa_value_with_gamma_and_preconditioner(C):
         g, pws, area = (_t(rng.uniform(0, 3, k).astype(np.float32)) for k in (2 * n, n, n))
         lam = torch.tensor([0.37], device="cuda")
         want = g.view(2, n) / (pws + 1.0 * lam * area).clamp(min=1.0)
-        C.precondition(g, pws, area, lam, 1.0)
+        assert C.precondition(g, pws, area, lam, 1.0)
         assert torch.equal(g, want.reshape(-1))
 
 
@@ -114,3 +114,30 @@ def test_force_in_node_order(C, nm, nf, fixed):
     want = C.scatter_pairs_to_nodes(force_o, order, count, n)
     got = C.electric_force_nodes(g, ex, ey, xy, order, rec, ratio, nm, nf, n, 0.0, 0.0, 1.0, 1.0, b, b, -1.0)
     assert torch.equal(got, want)
+
+
+def test_precondition_takes_what_the_tensor_expression_takes(C):
+    """Operands the kernel has no form for (a strided or fp64 node area, a pin
+    weight sum of another type, a lambda on the host) go through the tensor
+    expression; both count as a change of the gradient in place."""
+    from types import SimpleNamespace
+    from dreamplace_b200.place_obj import PreconditionOp
+    rng = np.random.RandomState(5)
+    n = 777
+    pws, area, g0 = (_t(rng.uniform(0, 3, k).astype(np.float32)) for k in (n, n, 2 * n))
+    lam = torch.tensor([0.37], device="cuda")
+    wide = torch.zeros(2 * n, device="cuda")
+    wide[::2] = area
+    want = (g0.view(2, n) / (pws + 1.0 * lam * area).clamp(min=1.0)).reshape(-1)
+    forms = {"kernel": (pws, area, lam, 0), "strided area": (pws, wide[::2], lam, 0),
+             "fp64 area": (pws, area.double(), lam, 1e-6), "fp64 pin weights": (pws.double(), area, lam, 1e-6),
+             "strided pin weights": (torch.stack([pws, pws], 1)[:, 0], area, lam, 0),
+             "host lambda": (pws, area, torch.tensor(0.37), 0)}
+    for name, (p, a, w, tol) in forms.items():
+        op = PreconditionOp(SimpleNamespace(num_nodes=n), SimpleNamespace(node_areas=a, net_weights=None),
+                            SimpleNamespace(pws_op=lambda _: p))
+        g = g0.clone()
+        version = g._version
+        assert op(g, w) is g and op.iteration == 1
+        assert g._version > version, name
+        assert float((g - want).abs().max()) <= tol * float(want.abs().max()), name
