@@ -163,21 +163,36 @@ __global__ void __launch_bounds__(256) pin_pos_forward_kernel(
 }
 
 // One warp per tile of 32 consecutive segments (a node's pins, a net's pins)
-// of a CSR: the tile's entries [p0, p1) are one contiguous range, gathered
-// kFoldPins at a time into the warp's buffer with four independent gathers a
-// lane, and each lane folds its own segment's entries [my0, my1) in order.  A
-// thread walking its own segment instead has one dependent gather in flight,
-// at an address no neighbour shares.  With the gathers of the other pin kernels
-// four to a thread it took a wirelength call at 7.1M pins from 256 to 245 us:
-// what bounds the node sums then is L2 sectors (69% of the memory pipe, two
-// sectors for a pin's 8 bytes), 72 us.
+// of a CSR.  A tile whose segments all count and whose starts ascend is one
+// contiguous range of entries [p0, p1), gathered kFoldPins at a time into the
+// warp's buffer with four independent gathers a lane, and each lane folds its
+// own segment's entries [my0, my1) in order.  In any other tile (a masked net,
+// whose entries are not to be read, or a start below the one before it) each
+// lane walks its own segment; the order of its sum is the same.  A thread
+// walking its own segment has one dependent gather in flight, at an address no
+// neighbour shares.  With the gathers of the other pin kernels four to a thread
+// the staged form took a wirelength call at 7.1M pins from 256 to 245 us: what
+// bounds the node sums then is L2 sectors (69% of the memory pipe, two sectors
+// for a pin's 8 bytes), 72 us.  HPWL of 2.2M nets, staged / walked, us: no net
+// masked 63 / 68, 3% masked (most tiles walk) 64 / 68, 30% 64 / 51; a masked net
+// of 8M pins 116,000 where its tile is staged, 38 walked.
 constexpr int kFoldThreads = 256;
 constexpr int kFoldPins = 128;
 
+// All lanes of the warp call it; `on`: the lane's segment counts.
 template <typename Fold>
 __device__ __forceinline__ void warp_fold(float2* stage, const int* __restrict__ flat, const float* __restrict__ px,
-                                          const float* __restrict__ py, int lane, int p0, int p1, int my0, int my1,
+                                          const float* __restrict__ py, int lane, int cnt, bool on, int my0, int my1,
                                           Fold fold) {
+  if (!__all_sync(0xffffffffu, lane >= cnt || (on && my0 <= my1))) {
+    if (on)
+      for (int k = my0; k < my1; ++k) {
+        const int id = __ldg(flat + k);
+        fold(make_float2(__ldg(px + id), __ldg(py + id)));
+      }
+    return;
+  }
+  const int p0 = __shfl_sync(0xffffffffu, my0, 0), p1 = __shfl_sync(0xffffffffu, my1, cnt - 1);
   for (int c0 = p0; c0 < p1; c0 += kFoldPins) {
     int id[kFoldPins / 32];
     float2 q[kFoldPins / 32];
@@ -211,9 +226,9 @@ __global__ void __launch_bounds__(kFoldThreads) pin_pos_backward_kernel(
     float sx = 0.f, sy = 0.f;
     const int cnt = min(num_physical - n0, 32);  // nodes of the tile with pins (warp-uniform)
     if (cnt > 0) {
-      const int my0 = i < num_physical ? node_start[i] : 0, my1 = i < num_physical ? node_start[i + 1] : 0;
-      const int p0 = __shfl_sync(0xffffffffu, my0, 0), p1 = __shfl_sync(0xffffffffu, my1, cnt - 1);
-      warp_fold(stage[threadIdx.x >> 5], flat_node2pin, gpx, gpy, lane, p0, p1, my0, my1, [&](float2 v) {
+      const bool on = i < num_physical;
+      const int my0 = on ? node_start[i] : 0, my1 = on ? node_start[i + 1] : 0;
+      warp_fold(stage[threadIdx.x >> 5], flat_node2pin, gpx, gpy, lane, cnt, on, my0, my1, [&](float2 v) {
         sx = fadd(sx, v.x);
         sy = fadd(sy, v.y);
       });
@@ -242,9 +257,8 @@ __global__ void __launch_bounds__(kFoldThreads) hpwl_kernel(const float* __restr
     const int my0 = live ? netpin_start[i] : 0, my1 = live ? netpin_start[i + 1] : 0;
     const bool on = live && net_mask[i];
     const float w = on && net_weights ? net_weights[i] : 1.f;
-    const int p0 = __shfl_sync(0xffffffffu, my0, 0), p1 = __shfl_sync(0xffffffffu, my1, cnt - 1);
     float max_x = -FLT_MAX, min_x = FLT_MAX, max_y = -FLT_MAX, min_y = FLT_MAX;
-    warp_fold(stage[threadIdx.x >> 5], flat_netpin, px, py, lane, p0, p1, my0, my1, [&](float2 v) {
+    warp_fold(stage[threadIdx.x >> 5], flat_netpin, px, py, lane, cnt, on, my0, my1, [&](float2 v) {
       min_x = fminf(min_x, v.x);
       max_x = fmaxf(max_x, v.x);
       min_y = fminf(min_y, v.y);

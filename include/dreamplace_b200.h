@@ -340,13 +340,15 @@ int dp_wa_merged_backward(const float* grad_pos, const int* pin2net_map,
 int dp_pin_pos_forward(const float* pos, int num_nodes, const float* pin_offset_x,
                        const float* pin_offset_y, const int* pin2node_map, int num_pins,
                        float* pin_pos, dp_stream_t stream);
-/* pin_pos/src/pin_pos_cuda_kernel.cu:50-74: node grad = sum of its pins' grads */
+/* pin_pos/src/pin_pos_cuda_kernel.cu:50-74: node grad = sum of its pins' grads,
+ * in the order of its segment [start[i], start[i + 1]) of flat_node2pin_map */
 int dp_pin_pos_backward(const float* grad_pin_pos, int num_pins,
                         const int* flat_node2pin_map, const int* flat_node2pin_start_map,
                         int num_physical_nodes, int num_nodes, float* grad_pos,
                         dp_stream_t stream);
 /* hpwl/src/hpwl_cuda_kernel.cu:10-39 (net-by-net); out_f64 holds DP_REDUCE_DOUBLES
- * doubles, [0] = fixed-order fp64 total; out_f32 optional */
+ * doubles, [0] = fixed-order fp64 total; out_f32 optional.  A masked net's
+ * entries of flat_netpin are not read. */
 int dp_hpwl(const float* pin_pos, int num_pins, const int* flat_netpin,
             const int* netpin_start, int num_nets, const float* net_weights,
             const unsigned char* net_mask, double* out_f64, float* out_f32,

@@ -141,3 +141,43 @@ def test_precondition_takes_what_the_tensor_expression_takes(C):
         assert op(g, w) is g and op.iteration == 1
         assert g._version > version, name
         assert float((g - want).abs().max()) <= tol * float(want.abs().max()), name
+
+
+def test_folds_read_only_the_segments_they_are_given(C):
+    """Segment i is [start[i], start[i + 1]), empty where the second is not above
+    the first, also for a start array that does not ascend; and a masked net's
+    entries are not read, however many it has."""
+    rng = np.random.RandomState(11)
+    P, n = 640, 45
+    xy = rng.uniform(-50, 50, 2 * P).astype(np.float32)
+    flat = rng.permutation(P).astype(np.int32)
+    for start in (np.array([5, 8, 0, 5], np.int32), rng.randint(0, P, n + 1).astype(np.int32)):
+        S = len(start) - 1
+        got = C.pin_pos_backward(_t(xy), torch.zeros(2 * S, device="cuda"), _t(flat), _t(start), S).cpu().numpy()
+        want, total = np.zeros(2 * S, np.float32), 0.0
+        mask = start[1:] > start[:-1]
+        for i in range(S):
+            px, py = (xy[a + flat[start[i]:max(start[i + 1], start[i])]] for a in (0, P))
+            for k in range(len(px)):
+                want[i] = np.float32(want[i] + px[k])
+                want[S + i] = np.float32(want[S + i] + py[k])
+            if mask[i]:
+                total += float(np.float32(np.float32(np.float32(px.max() - px.min()) + py.max()) - py.min()))
+        assert np.array_equal(got, want)
+        h = C.hpwl_forward(_t(xy), _t(flat), _t(start), torch.empty(0, device="cuda"), _t(mask.astype(np.uint8)))
+        assert abs(h[0].item() - total) <= 1e-13 * S * max(total, 1.0)  # fp64 sums in two orders
+    # one masked net of 8M entries among small ones: a warp that walks them needs
+    # 64k dependent rounds of L2 reads (over 30 ms), the rest of the call microseconds
+    big = 8 << 20
+    start = np.concatenate([np.arange(0, 80, 4), [big], big + np.arange(4, 44, 4)]).astype(np.int32)
+    flat = torch.arange(int(start[-1]), dtype=torch.int32, device="cuda") % 1000
+    mask = np.diff(start) < 100
+    args = (_t(rng.uniform(0, 9, 2 * int(start[-1])).astype(np.float32)), flat, _t(start),
+            torch.empty(0, device="cuda"), _t(mask.astype(np.uint8)))
+    C.hpwl_forward(*args)
+    t0, t1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    t0.record()
+    C.hpwl_forward(*args)
+    t1.record()
+    t1.synchronize()
+    assert t0.elapsed_time(t1) < 5.0
