@@ -542,7 +542,7 @@ class ElectricPotentialOrderedFunction(Function):
         bsx, bsy = op.bin_size_x, op.bin_size_y
         density_map, cells = op.ordered_density_map(pos, op.num_filler_nodes, 1.0 / (bsx * bsy))
         ctx.op, ctx.cells, ctx.precision = op, cells, precision
-        ctx.num_nodes = pos.numel() // 2
+        ctx.sizes = op.num_movable_nodes, op.num_filler_nodes, pos.numel() // 2
         ctx.density_map = density_map
         if recompute_field:
             energy = torch.zeros(1, dtype=torch.float64, device=pos.device) if fast_mode else \
@@ -565,10 +565,9 @@ class ElectricPotentialOrderedFunction(Function):
             fx, fy, _ = poisson_solve(ctx.density_map, op.bin_size_x, op.bin_size_y, ctx.precision, True,
                                       fast=_fast_solve(ctx.precision, ctx.density_map))
         g = grad_pos.reshape(1).to(torch.float32)
-        output = C.electric_force_nodes(g, fx.view(-1), fy.view(-1), xy_o, order, rec4, ratio_o,
-                                        op.num_movable_nodes, op.num_filler_nodes, ctx.num_nodes, float(op.xl),
-                                        float(op.yl), float(op.bin_size_x), float(op.bin_size_y), op.num_bins_x,
-                                        op.num_bins_y, -1.0)
+        output = C.electric_force_nodes(g, fx.view(-1), fy.view(-1), xy_o, order, rec4, ratio_o, *ctx.sizes,
+                                        float(op.xl), float(op.yl), float(op.bin_size_x), float(op.bin_size_y),
+                                        op.num_bins_x, op.num_bins_y, -1.0)
         return output, None, None, None, None
 
 

@@ -206,3 +206,24 @@ def test_trial_start_zeroes_large_maps_of_few_nodes(C):
     t1.record()
     t1.synchronize()
     assert t0.elapsed_time(t1) < 2.0
+
+
+def test_backward_serves_the_cells_of_its_forward(C):
+    """The filler count is an attribute that a program may set between calls (a
+    visiting order is kept for each): a backward still writes the force of the
+    cells that its own forward scattered."""
+    from dreamplace_b200 import synthetic
+    from dreamplace_b200.electric_potential import ElectricPotential
+    d = synthetic.scaled(2000, num_bins=64, seed=5)
+    centers = [_t(d.bin_centers(lo, hi, size)) for lo, hi, size in ((d.xl, d.xh, d.bin_size_x),
+                                                                    (d.yl, d.yh, d.bin_size_y))]
+    m = d.num_movable_nodes
+    op = ElectricPotential(_t(d.node_size_x), _t(d.node_size_y), *centers, d.target_density, d.xl, d.yl, d.xh, d.yh,
+                           d.bin_size_x, d.bin_size_y, m, d.num_terminals, d.num_filler_nodes, 0, True,
+                           _t(np.argsort(d.node_size_x[:m], kind="stable").astype(np.int32)), precision="fp32")
+    pos = _t(np.random.RandomState(2).uniform(0, d.xh * 0.9, 2 * d.num_nodes).astype(np.float32)).requires_grad_(True)
+    want, = torch.autograd.grad(op(pos), pos)
+    energy, fillers = op(pos), op.num_filler_nodes
+    op.num_filler_nodes = 0
+    got, = torch.autograd.grad(energy, pos)
+    assert fillers > 0 and torch.equal(got, want)
