@@ -323,64 +323,63 @@ def _graph_time(fn, reps=20):
     return s.elapsed_time(e) / reps
 
 
+def solve_work(M, N, prec, fast):
+    """(work, bound) of one Poisson solve: the products' flops (three 2-D
+    transforms, x3 for split-BF16; the energy is summed in the spectral domain),
+    or the maps that fast transforms read and write, each once."""
+    from dreamplace_b200.electric_potential import poisson_flops
+    return (12.0 * M * N, "hbm") if fast else (poisson_flops(M, N, prec), "tensor" if prec else "fp32")
+
+
 def piece_work(design, eng):
     """Algorithmic bytes (or flops) of each piece of one Nesterov trial, per
     launch (n_s scattered cells, P pins, E nets, n nodes, M x N bins):
 
     * density_scatter: 28 B per scattered cell (16 B record + 4 B ratio + 8 B
       position); per bin 4 B initial map read and the two maps written (the
-      movable-only map for the overflow and the movable + filler map);
-    * poisson_gemms: the GEMM flops of one solve (three 2-D transforms, x3
-      for split-BF16; the energy is summed in the spectral domain);
+      movable-only map for the overflow and the movable + filler map), and
+      4 B of hi + lo bf16 operand where the split-BF16 products read it;
+    * poisson_gemms: solve_work of the form the trial runs;
     * field_gather: per cell the same 28 B as the scatter + 8 B force written;
       per bin the two field maps read once;
     * wa_forward (HPWL included): per pin 12 B of pin arrays (node id, two
       offsets) + 8 B gradient written; per net 4 B start + 2 x 1 B masks +
       4 B weight; per node 8 B position (the pins' position gathers hit
       those 8 B);
-    * assemble_precondition: per pin 8 B gradient read; per node 4 B pin
-      start + 4 B inverse order + 8 B force + 4 B pin weight sum + 4 B area +
-      3 x 8 B (v_new, v, g) read + 8 B written;
+    * assemble_precondition (the trial's finish included): per pin 8 B gradient
+      read; per node 4 B pin start + 4 B inverse order + 8 B force + 4 B pin
+      weight sum + 4 B area + 3 x 8 B (v_new, v, g) read + 8 B written;
     * nesterov_trial: per node 3 x 8 B read (v, g, u) + 8 B cell size, 2 x 8 B
       written (u, v) + 8 B interleaved copy; per scattered cell 4 B order
       index + 8 B visiting-order copy written (the gather's re-read of the
-      interleaved copy is not counted)."""
-    from dreamplace_b200.electric_potential import poisson_flops
+      interleaved copy is not counted); per bin the two sums zeroed (4 B each,
+      8 B in fixed point)."""
     d, ep = design, eng.ep
     n_s = d.num_movable_nodes + d.num_filler_nodes
     M, N = ep.num_bins_x, ep.num_bins_y
     P, E, n = d.num_pins, d.num_nets, d.num_nodes
-    return {"density_scatter": (28.0 * n_s + 12.0 * M * N, "hbm"),
-            "poisson_gemms": (poisson_flops(M, N, eng.prec), "tensor" if eng.prec else "fp32"),
+    fast = eng.poisson_ws.fft_work is not None
+    return {"density_scatter": (28.0 * n_s + (16.0 if eng.prec == 3 and not fast else 12.0) * M * N, "hbm"),
+            "poisson_gemms": solve_work(M, N, eng.prec, fast),
             "field_gather": (36.0 * n_s + 8.0 * M * N, "hbm"),
             "wa_forward": (20.0 * P + 10.0 * E + 8.0 * n, "hbm"),
             "assemble_precondition": (8.0 * P + 64.0 * n, "hbm"),
-            "nesterov_trial": (56.0 * n + 12.0 * n_s, "hbm")}
+            "nesterov_trial": (56.0 * n + 12.0 * n_s + (16.0 if eng.det else 8.0) * M * N, "hbm")}
 
 
 def kernel_roofline(placer, design, peaks, reps=20):
-    """Device time of each piece of one Nesterov trial of the engine, each piece
-    graph-captured alone and replayed (warm L2), with its algorithmic work
-    (piece_work)."""
-    from dreamplace_b200.electric_potential import poisson_solve
+    """Device time of each piece of one Nesterov trial of the engine, as the trial
+    launches it (GPEngine.trial_pieces), graph-captured alone and replayed (warm
+    L2), with its algorithmic work (piece_work)."""
     eng = placer.stepper.eng
-    ep = eng.ep
     work = piece_work(design, eng)
     p = eng.slot
-    q = eng.next_slot(p)
-    v, g = eng.V[p], eng.G[p]
-    vn, gn = eng.V[q], eng.G[q]
-    torch.cuda.synchronize()  # the iteration enqueued ahead writes the slot after q
+    torch.cuda.synchronize()  # the iteration enqueued ahead writes the slot after p
     saved = eng.S[p].clone()
-    t = {}
-    t["density_scatter"] = _graph_time(lambda: eng.scatter_maps(v, eng.O[q]), reps)
-    rho = eng.dmap.mul(1.0 / (ep.bin_size_x * ep.bin_size_y))
-    t["poisson_gemms"] = _graph_time(lambda: poisson_solve(rho, ep.bin_size_x, ep.bin_size_y, eng.prec), reps)
-    ex, ey, _ = poisson_solve(rho, ep.bin_size_x, ep.bin_size_y, eng.prec)
-    t["field_gather"] = _graph_time(lambda: eng.field_force(v, ex, ey), reps)
-    t["wa_forward"] = _graph_time(lambda: eng.wirelength(v, eng.H[q]), reps)
-    t["assemble_precondition"] = _graph_time(lambda: eng.assemble(v, g, vn, gn), reps)
-    t["nesterov_trial"] = _graph_time(lambda: eng.nesterov_trial_only(p), reps)
+    pieces = eng.trial_pieces(p)
+    for fn in pieces.values():  # one trial: every piece then runs on its inputs
+        fn()
+    t = {k: _graph_time(fn, reps) for k, fn in pieces.items()}
     eng.S[p].copy_(saved)
     return {k: (t[k],) + work[k] for k in t}
 
@@ -393,12 +392,13 @@ def dropin_ops(placer, design, peaks, precision, reps=10):
     eager calls after one warm call.  Algorithmic bytes: the electric potential
     reads 28 B per scattered cell twice (scatter, gather) and writes 8 B of
     force, plus the bin maps (4 B init read, two 4 B maps written, two 4 B
-    field maps read); the Poisson GEMMs are counted as flops.  WA: pin_pos
+    field maps read); the products of the Poisson solve, where it runs them, are
+    counted as flops.  WA: pin_pos
     reads 8 B per node and 12 B per pin (node id, offsets) and writes 8 B per
     pin; WA reads 8 B and writes 8 B per pin gradient, plus 10 B per net;
     the backward sums 8 B per pin into 8 B per node."""
     import numpy as np
-    from dreamplace_b200.electric_potential import ElectricPotential, poisson_flops
+    from dreamplace_b200.electric_potential import ElectricPotential, fast_solve, poisson_flops
     from dreamplace_b200.placement_ops import PinPos
     from dreamplace_b200.weighted_average_wirelength import WeightedAverageWirelength
     from dreamplace_b200._native import precision_code
@@ -437,8 +437,10 @@ def dropin_ops(placer, design, peaks, precision, reps=10):
             pos.grad = None
             ep(pos).backward()
         ms = time_fn(ep_step)
+        fast = fast_solve(precision_code(precision), ep.initial_density_map)
         out["electric_potential_" + ("deterministic" if det else "fp32_atomic")] = {
-            "ms": round(ms, 4), "hbm_bytes": ep_bytes, "gemm_flop": poisson_flops(M, N, precision_code(precision)),
+            "ms": round(ms, 4), "hbm_bytes": ep_bytes,
+            "gemm_flop": 0.0 if fast else poisson_flops(M, N, precision_code(precision)),
             "achieved_gbs_if_hbm_only": round(ep_bytes / (ms * 1e-3) / 1e9, 1)}
         del ep
     deg = np.diff(d.flat_net2pin_start_map)

@@ -233,7 +233,7 @@ def poisson_solve(rho, bin_size_x, bin_size_y, precision, fast_mode=False, rho_s
 FAST_SPLIT_SIDE = 512
 
 
-def _fast_solve(precision, rho):
+def fast_solve(precision, rho):
     """Whether a density operator's solve may take the fast transforms: a
     split_bf16 one up to 512 bins a side.  The products' own error grows with the
     grid (of the field of a nearly even density 5e-6 at 64 bins, 2e-5 at 256, up
@@ -502,11 +502,11 @@ class ElectricPotentialFunction(Function):
             # keep only rho; the backward recomputes the field maps
             energy = torch.zeros(1, dtype=torch.float64, device=pos.device) if fast_mode else \
                 poisson_energy(density_map, bin_size_x, bin_size_y, precision,
-                               _fast_solve(precision, density_map))
+                               fast_solve(precision, density_map))
             ctx.field_map_x = ctx.field_map_y = None
         else:
             ex, ey, energy = poisson_solve(density_map, bin_size_x, bin_size_y, precision, fast_mode,
-                                           fast=_fast_solve(precision, density_map))
+                                           fast=fast_solve(precision, density_map))
             ctx.field_map_x = ex
             ctx.field_map_y = ey
         if fast_mode:
@@ -522,7 +522,7 @@ class ElectricPotentialFunction(Function):
         fx, fy = ctx.field_map_x, ctx.field_map_y
         if fx is None:
             fx, fy, _ = poisson_solve(ctx.density_map, bsx, bsy, ctx.precision, True,
-                                      fast=_fast_solve(ctx.precision, ctx.density_map))
+                                      fast=fast_solve(ctx.precision, ctx.density_map))
         output = C.electric_force(g, nbx, nby, a, b, c, d, fx.view([-1]), fy.view([-1]),
                                   ctx.pos, sxc, syc, ox, oy, ratio, bcx, bcy, float(xl), float(yl), float(xh),
                                   float(yh), float(bsx), float(bsy), int(nm), int(nf),
@@ -546,11 +546,11 @@ class ElectricPotentialOrderedFunction(Function):
         ctx.density_map = density_map
         if recompute_field:
             energy = torch.zeros(1, dtype=torch.float64, device=pos.device) if fast_mode else \
-                poisson_energy(density_map, bsx, bsy, precision, _fast_solve(precision, density_map))
+                poisson_energy(density_map, bsx, bsy, precision, fast_solve(precision, density_map))
             ctx.field_map_x = ctx.field_map_y = None
         else:
             ex, ey, energy = poisson_solve(density_map, bsx, bsy, precision, fast_mode,
-                                           fast=_fast_solve(precision, density_map))
+                                           fast=fast_solve(precision, density_map))
             ctx.field_map_x, ctx.field_map_y = ex, ey
         if fast_mode:
             return torch.zeros(1, dtype=pos.dtype, device=pos.device)
@@ -563,7 +563,7 @@ class ElectricPotentialOrderedFunction(Function):
         fx, fy = ctx.field_map_x, ctx.field_map_y
         if fx is None:
             fx, fy, _ = poisson_solve(ctx.density_map, op.bin_size_x, op.bin_size_y, ctx.precision, True,
-                                      fast=_fast_solve(ctx.precision, ctx.density_map))
+                                      fast=fast_solve(ctx.precision, ctx.density_map))
         g = grad_pos.reshape(1).to(torch.float32)
         output = C.electric_force_nodes(g, fx.view(-1), fy.view(-1), xy_o, order, rec4, ratio_o, *ctx.sizes,
                                         float(op.xl), float(op.yl), float(op.bin_size_x), float(op.bin_size_y),

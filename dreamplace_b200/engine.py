@@ -424,61 +424,118 @@ class GPEngine(object):
         C.precondition_step_size(g, g_ref, v_new, v_ref, self._pws(), self.data.node_areas,
                                  self.model.density_weight, self.S[self.slot])
 
-    def objective_and_step(self, v, g, v_new, g_new, s):
-        """The trial's objective at v_new and its preconditioned gradient into g_new,
-        with the fp64 step-size norms against (v, g) into slot s's scalars: the
-        field force is gathered in visiting order and assembled per node together
-        with the wirelength pin sum, the preconditioner and the norms (one pass
-        over the nodes).  The HPWL and overflow of v_new land in the metric
-        buffers of slot s + 1.  dp_trial_start has zeroed the density sums and
-        the energy; dp_trial_finish ends every sum and fills the metrics row,
-        also the host's."""
-        ep, dc, d = self.ep, self.data, self.design
-        q_new = (s + 1) % NSLOT
-        w = self.weights[s]
+    # the trial's pieces (PIECES), each what a trial from slot s into slot s + 1
+    # launches for it; dp_trial_finish ends the sums of three of them
+    def _start_piece(self, s, head):
+        d, t, r = self.design, (s + 1) % NSLOT, (s - 1) % NSLOT
+        scatter_write = self.xyo_mode == "trial"
+        zero = [self.scratch2] if self.det else [self.omap, self.dmap]
+        C.trial_start([self.S[r], self.sched[r], self.sched[s], self.H[r][0:1], self.O[r][0:1], self.weights[r],
+                       self.weights[s]] if head else None, self.head_scalars,
+                      self.gate if self.use_graphs else None, self.V[s], self.G[s], self.U[s], self.U[t], self.V[t],
+                      self.XY[t], self.S[s], self.data.node_size_x, self.data.node_size_y, float(d.xl), float(d.yl),
+                      float(d.xh), float(d.yh), d.num_movable_nodes, d.num_filler_nodes,
+                      self.inv_order if scatter_write else None, self.XYO[t] if scatter_write else None, zero,
+                      self.poisson_ws.energy, self.O[t][2:3])
+        if self.xyo_mode == "gather":
+            C.gather_order_xy(self.XY[t], self.order, self.order.numel(), self.XYO[t])
+
+    def _wirelength_piece(self, s):
+        """Returns the block count of the WA and HPWL sums."""
+        dc, t = self.data, (s + 1) % NSLOT
+        return C.trial_wirelength(self.xy(self.V[t]), self.group_deg, self.group_base, self.group_net, self.ln_node,
+                                  self.ln_offx, self.ln_offy, self.ln_csr if self.lane_of_csr is None else None,
+                                  dc.net_weights, dc.net_mask_ignore_large_degrees, self.weights[s][2:3],
+                                  self.wl64_buf, self.gnode, dc.net_mask_all, self.H[t])
+
+    def _density_piece(self, s):
+        """Returns the block count of the overflow's sum."""
+        ep, t = self.ep, (s + 1) % NSLOT
+        xy_o, order = self._cells_xy(self.V[t])
+        # the products read the map as a hi + lo bf16 operand, which the pass that
+        # finishes the map then writes too
+        op = self.poisson_ws.rho if self.prec == 3 and self.poisson_ws.fft_work is None else None
+        return C.trial_density(xy_o, order, self.rec4, self.ratio_o, ep.num_movable_nodes, self.order.numel(),
+                               ep.initial_density_map.view(-1), float(ep.xl), float(ep.yl), float(ep.xh),
+                               float(ep.yh), float(ep.bin_size_x), float(ep.bin_size_y), ep.num_bins_x,
+                               ep.num_bins_y, int(self.det), self.scratch2, self.omap.view(-1), self.dmap.view(-1),
+                               op.hi if op is not None else None, op.lo if op is not None else None,
+                               self.ovf_target, self.O[t])
+
+    def _solve_piece(self):
+        """The solve of self.dmap; returns (ex, ey, energy), the workspace's."""
+        ep = self.ep
+        if self.prec not in (0, 3) and self.poisson_ws.fft_work is None:
+            self.poisson_ws.rho.fill(self.dmap)
+        # rho = D / bin area is applied as the first GEMM's alpha
+        return poisson_solve(self.dmap, ep.bin_size_x, ep.bin_size_y, self.prec, bool(ep.fast_mode),
+                             1.0 / (ep.bin_size_x * ep.bin_size_y), self.poisson_ws, prepared=True)
+
+    def _force_piece(self, s, ex, ey, energy):
+        ep = self.ep
+        xy_o, order = self._cells_xy(self.V[(s + 1) % NSLOT])
+        C.trial_force(energy, self.weights[s][0:1], self.factor_quad, ex.view(-1), ey.view(-1), xy_o, order,
+                      self.rec4, self.ratio_o, self.order.numel(), float(ep.xl), float(ep.yl), float(ep.bin_size_x),
+                      float(ep.bin_size_y), ep.num_bins_x, ep.num_bins_y, -1.0, self.force_o)
+
+    def _assemble_piece(self, s, wa_blocks, ovf_blocks, energy):
+        """The preconditioned gradient and the step-size norms, the end of every
+        sum, the step-size test and the metrics row: HPWL / overflow of v_k
+        (computed when v_k was the trial point) and the trial's scalars, on the
+        device and in the host's pinned copy."""
+        d, dc, t, w = self.design, self.data, (s + 1) % NSLOT, self.weights[s]
+        norm_blocks = C.trial_assemble(self.gnode, self.node_start, self.one, self.force_o, self.inv_order,
+                                       d.num_movable_nodes, d.num_filler_nodes, self._pws(), dc.node_areas, w[0:1],
+                                       self.V[t], self.V[s], self.G[s], self.G[t], self.S[s], self.lane_of_csr)
+        C.trial_finish(self.wl64_buf, self.H[t], wa_blocks, self.O[t], ovf_blocks, self.ovf_area, energy, w[0:1],
+                       self.factor_quad, self.S[s], norm_blocks, self.H[s], self.O[s], self.obj64, self.metrics[s],
+                       self.metrics_dev[s])
+
+    def trial_pieces(self, s):
+        """{piece: function that launches it alone} for a trial from slot s, for
+        timing and profiling: run in order they are a trial.  The scatter adds onto
+        what the start zeroed, so the maps of a repeated one are not densities.  The
+        next step enqueues its trial afresh; the caller restores S[s]."""
+        head = self.iterations > 0
+        self.enqueued = None
+        sums = {}
+
+        def wirelength():
+            sums["wa"] = self._wirelength_piece(s)
+
+        def density():
+            sums["ovf"] = self._density_piece(s)
+        ws = self.poisson_ws
+        return {"nesterov_trial": lambda: self._start_piece(s, head), "wa_forward": wirelength,
+                "density_scatter": density, "poisson_gemms": self._solve_piece,
+                "field_gather": lambda: self._force_piece(s, ws.ex, ws.ey, ws.energy),
+                "assemble_precondition": lambda: self._assemble_piece(s, sums["wa"], sums["ovf"], ws.energy)}
+
+    def objective_and_step(self, s):
+        """The trial's objective at the trial point and its preconditioned gradient
+        into slot s + 1, with the fp64 step-size norms against slot s: the field
+        force is gathered in visiting order and assembled per node together with
+        the wirelength pin sum, the preconditioner and the norms (one pass over the
+        nodes).  The HPWL and overflow of the trial point land in the metric
+        buffers of slot s + 1.  dp_trial_start has zeroed the density sums and the
+        energy."""
         # (the WA forward was also run on a second stream beside the density
         # chain: its kernels and the scatter's, or the GEMMs', slow each other
         # down by about what they would overlap, ~1% net, so it runs in line)
         self._mark("wa_forward", 0)
-        wa_blocks = C.trial_wirelength(self.xy(v_new), self.group_deg, self.group_base, self.group_net, self.ln_node,
-                                       self.ln_offx, self.ln_offy,
-                                       self.ln_csr if self.lane_of_csr is None else None, dc.net_weights,
-                                       dc.net_mask_ignore_large_degrees, w[2:3], self.wl64_buf, self.gnode,
-                                       dc.net_mask_all, self.H[q_new])
+        wa_blocks = self._wirelength_piece(s)
         self._mark("wa_forward", 1)
         self._mark("density_scatter", 0)
-        xy_o, order = self._cells_xy(v_new)
-        # the solve's first product reads the map as a hi + lo bf16 operand, which
-        # the pass that finishes the map then writes too
-        op = self.poisson_ws.rho if self.prec == 3 and self.poisson_ws.fft_work is None else None
-        ovf_blocks = C.trial_density(xy_o, order, self.rec4, self.ratio_o, ep.num_movable_nodes, self.order.numel(),
-                                     ep.initial_density_map.view(-1), float(ep.xl), float(ep.yl), float(ep.xh),
-                                     float(ep.yh), float(ep.bin_size_x), float(ep.bin_size_y), ep.num_bins_x,
-                                     ep.num_bins_y, int(self.det), self.scratch2, self.omap.view(-1),
-                                     self.dmap.view(-1), op.hi if op is not None else None,
-                                     op.lo if op is not None else None, self.ovf_target, self.O[q_new])
+        ovf_blocks = self._density_piece(s)
         self._mark("density_scatter", 1)
         self._mark("poisson_gemms", 0)
-        if op is None and self.poisson_ws.fft_work is None and self.prec != 0:
-            self.poisson_ws.rho.fill(self.dmap)
-        # rho = D / bin area is applied as the first GEMM's alpha
-        ex, ey, energy = poisson_solve(self.dmap, ep.bin_size_x, ep.bin_size_y, self.prec, bool(ep.fast_mode),
-                                       1.0 / (ep.bin_size_x * ep.bin_size_y), self.poisson_ws, prepared=True)
+        ex, ey, energy = self._solve_piece()
         self._mark("poisson_gemms", 1)
         self._mark("field_gather", 0)
-        C.trial_force(energy, w[0:1], self.factor_quad, ex.view(-1), ey.view(-1), xy_o, order, self.rec4,
-                      self.ratio_o, self.order.numel(), float(ep.xl), float(ep.yl), float(ep.bin_size_x),
-                      float(ep.bin_size_y), ep.num_bins_x, ep.num_bins_y, -1.0, self.force_o)
+        self._force_piece(s, ex, ey, energy)
         self._mark("field_gather", 1)
         self._mark("assemble_precondition", 0)
-        norm_blocks = C.trial_assemble(self.gnode, self.node_start, self.one, self.force_o, self.inv_order,
-                                       d.num_movable_nodes, d.num_filler_nodes, self._pws(), dc.node_areas, w[0:1],
-                                       v_new, v, g, g_new, self.S[s], self.lane_of_csr)
-        # the metrics row: HPWL / overflow of v_k (computed when v_k was the trial
-        # point) and the trial's scalars, on the device and in the host's pinned copy
-        C.trial_finish(self.wl64_buf, self.H[q_new], wa_blocks, self.O[q_new], ovf_blocks, self.ovf_area, energy,
-                       w[0:1], self.factor_quad, self.S[s], norm_blocks, self.H[s], self.O[s], self.obj64,
-                       self.metrics[s], self.metrics_dev[s])
+        self._assemble_piece(s, wa_blocks, ovf_blocks, energy)
         self._mark("assemble_precondition", 1)
         self.last_energy = energy
         return energy
@@ -616,24 +673,11 @@ class GPEngine(object):
         """One Nesterov trial from slot s into slot s + 1.  head: the first trial
         of an iteration k >= 1, preceded by the loop's between-iteration work on
         the device (advance, density weight, gamma from slot s - 1)."""
-        t = (s + 1) % NSLOT
         self._mark_slot = s
-        r = (s - 1) % NSLOT
-        d = self.design
-        scatter_write = self.xyo_mode == "trial"
-        zero = [self.scratch2] if self.det else [self.omap, self.dmap]
         self._mark("nesterov_trial", 0)
-        C.trial_start([self.S[r], self.sched[r], self.sched[s], self.H[r][0:1], self.O[r][0:1], self.weights[r],
-                       self.weights[s]] if head else None, self.head_scalars,
-                      self.gate if self.use_graphs else None, self.V[s], self.G[s], self.U[s], self.U[t], self.V[t],
-                      self.XY[t], self.S[s], self.data.node_size_x, self.data.node_size_y, float(d.xl), float(d.yl),
-                      float(d.xh), float(d.yh), d.num_movable_nodes, d.num_filler_nodes,
-                      self.inv_order if scatter_write else None, self.XYO[t] if scatter_write else None, zero,
-                      self.poisson_ws.energy, self.O[t][2:3])
-        if self.xyo_mode == "gather":
-            C.gather_order_xy(self.XY[t], self.order, self.order.numel(), self.XYO[t])
+        self._start_piece(s, head)
         self._mark("nesterov_trial", 1)
-        self.objective_and_step(self.V[s], self.G[s], self.V[t], self.G[t], s)
+        self.objective_and_step(s)
 
     def nesterov_trial_only(self, s):
         """The trial point from slot s into slot s + 1, and its visiting-order

@@ -4,58 +4,46 @@
 
 Runs global placement of a synthetic design (graph engine, split-BF16 Poisson
 solve, fp32 scatter) to the given iteration, refreshes the visiting order at
-the position reached, then runs the chosen piece ``--repeat`` times on it with
-a synchronize after each run, inside the NVTX range ``profile_piece``.  Under
-ncu, ``--nvtx --nvtx-include "profile_piece/" -k <kernel> -s 1 -c 1`` then
+the position reached, runs one trial piece by piece, then the chosen piece
+``--repeat`` times, as the trial launches it, with a synchronize after each run,
+inside the NVTX range ``profile_piece``.  Under ncu, ``--nvtx --nvtx-include "profile_piece/" -k <kernel> -s 1 -c 1`` then
 captures one warm launch of the piece's kernel.  Pieces:
 
 * ``wa``: WA forward + HPWL (``wa_lane_kernel``);
-* ``scatter``: the split density scatter (``tile_scatter_kernel``,
+* ``scatter``: the density scatter of both maps (``tile_scatter_kernel``,
   ``finish_maps_kernel``);
-* ``poisson``: the Poisson solve of the current density map (``tc_gemm_kernel``);
+* ``poisson``: the Poisson solve of the current density map: ``tc_gemm_kernel``,
+  or ``fft_rows_kernel`` and ``fft_cols_kernel`` where the trial solves by the
+  fast transforms (split-BF16 up to 128 bins a side);
 * ``field``: the field gather (``electric_force_records_kernel``);
-* ``assemble``: gradient assembly + preconditioner (``assemble_precondition_kernel``);
-* ``trial``: the Nesterov trial point (``nesterov_trial_kernel``).
+* ``assemble``: gradient assembly + preconditioner and the trial's end
+  (``assemble_precondition_kernel``, ``trial_finish_kernel``);
+* ``trial``: the Nesterov trial point and the zeroing (``trial_start_kernel``).
 """
 import argparse
 
 import torch
 
 from . import synthetic
-from .electric_potential import poisson_solve
 from .nonlinear_place import NonLinearPlace
 from .params import Params
 
-PIECES = ("wa", "scatter", "poisson", "field", "assemble", "trial")
+PIECES = {"wa": "wa_forward", "scatter": "density_scatter", "poisson": "poisson_gemms", "field": "field_gather",
+          "assemble": "assemble_precondition", "trial": "nesterov_trial"}
 
 
 def run_piece(eng, piece, repeat):
-    ep = eng.ep
     p = eng.slot
-    q = eng.next_slot(p)
-    v, g = eng.V[p], eng.G[p]
-    vn, gn = eng.V[q], eng.G[q]
     saved = eng.S[p].clone()
-    eng.scatter_maps(v, eng.O[q])
-    rho = eng.dmap.mul(1.0 / (ep.bin_size_x * ep.bin_size_y))
-    ex, ey, _ = poisson_solve(rho, ep.bin_size_x, ep.bin_size_y, eng.prec)
+    pieces = eng.trial_pieces(p)
+    for fn in pieces.values():  # one trial: every piece then runs on its inputs
+        fn()
     torch.cuda.synchronize()
     # the piece's launches sit in the NVTX range "profile_piece" (ncu --nvtx
     # --nvtx-include "profile_piece/" captures them and none of the GP run's)
     torch.cuda.nvtx.range_push("profile_piece")
     for _ in range(repeat):
-        if piece == "wa":
-            eng.wirelength(v, eng.H[q])
-        elif piece == "scatter":
-            eng.scatter_maps(v, eng.O[q])
-        elif piece == "poisson":
-            poisson_solve(rho, ep.bin_size_x, ep.bin_size_y, eng.prec)
-        elif piece == "field":
-            eng.field_force(v, ex, ey)
-        elif piece == "assemble":
-            eng.assemble(v, g, vn, gn)
-        elif piece == "trial":
-            eng.nesterov_trial_only(p)
+        pieces[PIECES[piece]]()
         torch.cuda.synchronize()
     torch.cuda.nvtx.range_pop()
     eng.S[p].copy_(saved)
@@ -63,7 +51,7 @@ def run_piece(eng, piece, repeat):
 
 def main(argv=None):
     ap = argparse.ArgumentParser(description=__doc__.split("\n\n")[0])
-    ap.add_argument("--piece", choices=PIECES, required=True)
+    ap.add_argument("--piece", choices=sorted(PIECES), required=True)
     ap.add_argument("--design", default="cells_2m", choices=["cells_10k", "cells_2m"])
     ap.add_argument("--iterations", type=int, default=1499, help="GP iterations run before the piece")
     ap.add_argument("--repeat", type=int, default=2)

@@ -324,3 +324,42 @@ def test_pinned_rows_outlive_the_warm_up_of_the_graphs(design):
     torch.cuda.synchronize()
     engine._release_retired()
     assert not any(kept is rows for kept, _ in engine._RETIRED)
+
+
+@pytest.mark.parametrize("bins,precision,launches,bound", [(128, "split_bf16", 3, "hbm"), (256, "split_bf16", 4, "tensor"),
+                                                          (256, "fp32", 3, "hbm"), (136, "fp32", 4, "fp32")])
+def test_timed_pieces_are_the_trials_own(bins, precision, launches, bound):
+    """GPEngine.trial_pieces (what the bench and the profiler time) run in order is
+    a trial, bit for bit, and its solve is the one that the trial runs: three
+    passes of the fast transforms, rated by their maps, or four products."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import bench
+    from dreamplace_b200._native import C
+    d = synthetic.scaled(3000, num_bins=bins, seed=9)
+    placer, _, _ = run(d, "graph", precision, 5, deterministic=1)
+    eng = placer.stepper.eng
+    torch.cuda.synchronize()
+    s = eng.slot
+    t = (s + 1) % 3
+    state = lambda: [eng.V[t].clone(), eng.U[t].clone(), eng.G[t].clone(), eng.S[s][:8].clone(),  # noqa: E731
+                     eng.metrics[s][:7].clone()]
+    eng._trial(s, head=True)
+    want = state()
+    for buf in (eng.V[t], eng.U[t], eng.G[t]):
+        buf.fill_(-1.0)
+    count = {}
+    for name, piece in eng.trial_pieces(s).items():
+        before = C.launch_count()
+        piece()
+        count[name] = C.launch_count() - before
+    got = state()
+    assert all(torch.equal(a, b) for a, b in zip(got[:4], want[:4]))
+    # the objective adds the energy, an atomic fp64 sum: its last bits vary
+    assert torch.allclose(got[4], want[4], rtol=1e-12, atol=0.0)
+    assert count["poisson_gemms"] == launches
+    assert bench.piece_work(d, eng)["poisson_gemms"][1] == bound
+    work = bench.kernel_roofline(placer, d, {}, reps=1)
+    assert set(work) == set(count) and all(ms > 0 for ms, _, _ in work.values())
+    eng.step()  # the engine goes on from slot s
+    assert all(torch.equal(a, b) for a, b in zip(state()[:3], want[:3]))
