@@ -1,19 +1,22 @@
 """Precision sweep of the Poisson solve.
 
-For transform sizes 512^2 .. 4096^2 and each solve precision (fp32, tf32,
-bf16, split-bf16) this measures
+For transform sizes 64^2 .. 4096^2 and each form of the solve -- the matrix
+products in fp32, tf32, bf16 and split-bf16, and the fast transforms, which
+serve fp32 and split-bf16 on these sizes (``fast``) -- this measures
 
-* the error of the field maps (max-norm relative) and of the energy against an
-  fp64 evaluation of the same matrix forms (the reference's dct2_fft2 /
-  idxst_idct / idct_idxst / idct2 scalings, electric_potential.py:504-519),
-* the device time of one solve (CUDA events over graph replays) and the GEMM
-  throughput it implies,
+* the error of the field maps (max-norm and 2-norm, relative) and of the energy
+  against an fp64 evaluation of the same matrix forms (the reference's
+  dct2_fft2 / idxst_idct / idct_idxst / idct2 scalings,
+  electric_potential.py:504-519),
+* the device time of one solve (CUDA events over graph replays), with the GEMM
+  throughput it implies for the products and, for the fast transforms, the rate
+  at which the maps it reads and writes move (each once: 12 bytes a bin),
 
 on density maps rasterised from the 10k-cell design's GP positions at
 iterations 0, 300 and 700; and with ``--gp`` the end-of-GP HPWL, overflow and
-iteration count of that design for each precision.
+iteration count of that design for each ``dct_precision``.
 
-Usage: python -m dreamplace_b200.precision_sweep [--sizes 512,1024,2048,4096] [--gp]
+Usage: python -m dreamplace_b200.precision_sweep [--sizes 64,128,...,4096] [--gp]
 Prints one JSON object per line.
 """
 import argparse
@@ -105,16 +108,22 @@ def sweep_sizes(design, snaps, sizes):
             dmap, bs = density_on_grid(design, pos, M)
             rho = (dmap / (bs * bs)).contiguous()
             rex, rey, renergy = fp64_solve(rho, bs)
-            for prec in PRECISIONS:
-                ex, ey, energy = poisson_solve(rho, bs, bs, prec)
+            for form in PRECISIONS + ("fast",):
+                fast = form == "fast"
+                solve = lambda: poisson_solve(rho, bs, bs, "fp32" if fast else form, fast=fast)  # noqa: E731,B023
+                ex, ey, energy = solve()
                 err = max(float((ex.double() - rex).abs().max() / rex.abs().max()),
                           float((ey.double() - rey).abs().max() / rey.abs().max()))
-                line = {"size": M, "gp_iteration": it, "precision": prec, "field_rel_err": err,
+                err2 = max(float((ex.double() - rex).norm() / rex.norm()), float((ey.double() - rey).norm() / rey.norm()))
+                line = {"size": M, "gp_iteration": it, "form": form, "field_rel_err": err, "field_rel_err_2norm": err2,
                         "energy_rel_err": abs(float(energy.item()) - renergy) / abs(renergy)}
                 if it == min(snaps):
-                    ms = graph_ms(lambda: poisson_solve(rho, bs, bs, prec))
-                    line.update(solve_ms=round(ms, 4),
-                                gemm_tflops=round(poisson_flops(M, M, prec) / (ms * 1e-3) / 1e12, 1))
+                    ms = graph_ms(solve)
+                    line.update(solve_ms=round(ms, 4))
+                    if fast:
+                        line.update(map_gbs=round(12.0 * M * M / (ms * 1e-3) / 1e9, 1))
+                    else:
+                        line.update(gemm_tflops=round(poisson_flops(M, M, form) / (ms * 1e-3) / 1e12, 1))
                 print(json.dumps(line), flush=True)
             del rex, rey
             torch.cuda.empty_cache()
@@ -131,7 +140,7 @@ def sweep_gp(design):
 
 def main(argv=None):
     ap = argparse.ArgumentParser(description=__doc__.split("\n")[0])
-    ap.add_argument("--sizes", default="512,1024,2048,4096")
+    ap.add_argument("--sizes", default="64,128,256,512,1024,2048,4096")
     ap.add_argument("--iterations", default="0,300,700")
     ap.add_argument("--gp", action="store_true", help="also run the full GP per precision")
     args = ap.parse_args(argv)
