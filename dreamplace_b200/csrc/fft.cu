@@ -11,10 +11,10 @@
 //               columns stay in shared memory between the three transforms
 //   3. rows:    Ex = 4 (.) Ch_N^T, Ey = 4 (.) Sh_N^T, one complex transform per row
 // against operand preparation and 4 GEMM launches of the dense form.  One solve,
-// us, split-BF16 products -> fast transforms (replayed graph): 64^2 26 -> 9,
-// 256^2 37 -> 10, 512^2 45 -> 13, 1024^2 68 -> 25, 2048^2 389 -> 63, 4096^2
-// 2800 -> 236; relative error of the field at 1024^2 against fp64 8e-7 (the
-// reference's fp32 spectral weights) instead of 1e-5.  Up to 512^2 the three
+// us, split-BF16 products -> fast transforms (replayed graph): 64^2 27 -> 11,
+// 256^2 36 -> 13, 512^2 46 -> 15, 1024^2 68 -> 25, 2048^2 389 -> 65, 4096^2
+// 2420 -> 243; relative error of the field (2-norm) at 1024^2 against fp64 4e-7
+// to 5e-7 on GP states, the products' 2e-5 to 4e-5.  Up to 512^2 the three
 // launches bound it, from 2048^2 issue and the exchanges (57% issue, 128 MB of
 // rows in 38 us = 3.4 TB/s at 4096^2); at 1024^2 the column pass's 128 blocks.
 //

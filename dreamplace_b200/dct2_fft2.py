@@ -1,10 +1,11 @@
-"""2-D DCT family of the Poisson solve, as GEMMs on the tensor cores.
+"""2-D DCT family of the Poisson solve, as fast transforms and as GEMMs on the tensor cores.
 
 Drop-in for the reference's ``dreamplace/ops/dct/dct2_fft2.py``: modules
 ``DCT2``, ``IDCT2``, ``IDCT_IDXST``, ``IDXST_IDCT`` taking ``(expkM, expkN)`` and
 transforming an ``M x N`` map with ``.forward(x)``.  The reference computes them
-with a real FFT and twiddle kernels (dct/src/dct2_fft2_cuda_kernel.cu); here each
-2-D transform is two dense products with cosine / sine matrices,
+with a real FFT and twiddle kernels (dct/src/dct2_fft2_cuda_kernel.cu); here, off
+the grids that the fast transforms below take, each 2-D transform is two dense
+products with cosine / sine matrices,
 
     dct2_fft2(x)   = 4/(M N) * C_M  x C_N^T      C_n[k,i] = cos(pi (2i+1) k / (2n))
     idct2_fft2(y)  = 4 * Ch_M y Ch_N^T          Ch_n[u,p] = w_p cos(pi p (u+1/2) / n),  w_0 = 1/2
@@ -20,9 +21,11 @@ On grids whose sides are powers of two from 64 to 4096, ``fp32`` and
 ``split_bf16`` (the two settings that ask for fp32-grade results) run as fast
 transforms in fp32 instead (csrc/fft.cu): fewer operations and one read and
 write of the map per axis, and closer to fp64 than either product.  Poisson
-solve, us, product -> fast transform: split_bf16 64^2 26 -> 9, 1024^2 68 -> 25,
-4096^2 2800 -> 236; fp32 64^2 49 -> 9, 1024^2 555 -> 25.  ``tf32`` and ``bf16``
-name the arithmetic of a product, and stay one.
+solve, us, product -> fast transform: split_bf16 64^2 27 -> 11, 1024^2 68 -> 25,
+4096^2 2420 -> 243; fp32 64^2 50 -> 11, 1024^2 556 -> 25.  ``tf32`` and ``bf16``
+name the arithmetic of a product, and stay one.  (A split_bf16 solve inside a
+density operator or a GP trial keeps the products on larger grids:
+electric_potential.fast_solve.)
 """
 
 import functools

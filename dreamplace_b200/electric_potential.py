@@ -18,10 +18,10 @@ the spectral weights in the epilogue, the two right products batched in one
 launch, and the two left products batched with the Ex/Ey stores.  The energy
 is summed in the spectral domain by the second launch's epilogue,
   sum_xy rho IDCT2(a winv) = M N sum_uv w_u w_v winv_uv a_uv^2 (w_0 = 1/2),
-so the potential map is never formed.  In fp32 and split_bf16 on power-of-two
-grids the solve runs as fast transforms in three launches instead
-(csrc/fft.cu, dct2_fft2.fft_serves): rows; columns, weights, energy and the
-inverse column transforms; rows.
+so the potential map is never formed.  On power-of-two grids the fp32 solve, and
+the split_bf16 one within the limits of ``fast_solve``, run as fast transforms in
+three launches instead (csrc/fft.cu, dct2_fft2.fft_serves): rows; columns,
+weights, energy and the inverse column transforms; rows.
 Backward: the hand-written adjoint ``-electric_force`` (reference :219-275).
 
 The modules (``ElectricOverflow``, ``ElectricPotential``) keep a spatial
@@ -230,17 +230,38 @@ def poisson_solve(rho, bin_size_x, bin_size_y, precision, fast_mode=False, rho_s
     return ex, ey, energy
 
 
-FAST_SPLIT_SIDE = 512
+# The rule of the solve, on the maps that fft_serves: fp32 takes the fast
+# transforms everywhere, tf32 and bf16 (which name a product's arithmetic)
+# nowhere; split_bf16 in poisson_solve and the transform modules everywhere, in a
+# density operator up to FAST_OPERATOR_SIDE bins a side and in a trial of the
+# graph engine up to FAST_TRIAL_SIDE.  Error of the field against 64 bits (2-norm,
+# relative) on the density of cells spread over the die, one a bin, and early in
+# placement (over 0.3 of its width), and a solve's time in a replayed graph:
+#
+#   bins a side                        64      128     256     512     1024
+#   split_bf16 products, spread out    9e-6    9e-6    2e-5    9e-5    4e-4
+#   split_bf16 products, early         6e-6    7e-6    9e-6    1e-5    1e-5
+#   fast transforms, either            3e-7    3e-7    3e-7    4e-7    4e-7
+#   products / fast transforms, us     27/11   33/13   36/13   46/15   68/25
+#
+# Error and time alone are for the fast transforms at every size.  The limits
+# keep large designs' results where the products have them: the two forms differ
+# by the products' error, which grows with the grid on an even density (whose
+# field is a small difference of large terms), and a trajectory multiplies it (16
+# iterations of 200k cells on 512 x 512 bins: 6e-3 of the gradient).  Up to 128
+# bins trials on the fast transforms stay about as close to trials with a 64-bit
+# solve as the products do (the gradient of two seeds each: 10k cells, 32
+# iterations, 6.3e-4 and 2.5e-4 away, the products 6.2e-4 and 2.8e-4; 16k cells, 8
+# iterations, 1.2e-5 and 1e-6 against 3e-6 and 8e-6; 3k cells on 64 bins 1.3e-5 and
+# 1.1e-5 against 1.8e-2 and 2.3e-5).
+FAST_OPERATOR_SIDE = 512
+FAST_TRIAL_SIDE = 128
 
 
-def fast_solve(precision, rho):
-    """Whether a density operator's solve may take the fast transforms: a
-    split_bf16 one up to 512 bins a side.  The products' own error grows with the
-    grid (of the field of a nearly even density 5e-6 at 64 bins, 2e-5 at 256, up
-    to 1e-3 at 1024, where it would show between the two); the fast transforms'
-    is 1e-7, and a call of the products is 5 launches and 10 allocations against
-    3 and 4."""
-    return precision_code(precision) != 3 or max(rho.shape) <= FAST_SPLIT_SIDE
+def fast_solve(precision, rho, side=FAST_OPERATOR_SIDE):
+    """Whether a solve of the map rho in a place with the limit ``side`` may take
+    the fast transforms (the rule above)."""
+    return precision_code(precision) != 3 or max(rho.shape) <= side
 
 
 class ElectricDensityMapFunction(Function):

@@ -30,7 +30,7 @@ import numpy as np
 import torch
 
 from ._native import C, precision_code
-from .electric_potential import PoissonWorkspace, poisson_solve
+from .electric_potential import FAST_TRIAL_SIDE, PoissonWorkspace, fast_solve, poisson_solve
 
 # device scalar slots of the optimizer state (gp_step.cu)
 NS_ALPHA, NS_A, NS_A_NEXT, NS_COEF, NS_ACC_DV, NS_ACC_DG, NS_ALPHA_NEW, NS_ACCEPT = range(8)
@@ -169,17 +169,10 @@ class GPEngine(object):
         self.scratch = self.scratch2[:bins] if self.det else None
         self.prec = precision_code(ep.precision)
         # the Poisson solve's operands and outputs, allocated once: every trial
-        # (eager or captured) of this design solves on its one stream.  split_bf16
-        # trials keep the matrix products: the fast transforms' field differs from
-        # theirs by the products' own error (1e-4 of the field of a nearly even
-        # density), which 16 iterations of a 200k-cell design turned into up to 6e-3
-        # of the gradient, and a run's trajectory is to stay what it was (a solve at
-        # 1024^2 takes 67 us instead of 25); the products' error falls with the square
-        # of the side, and up to 128 bins the fast transforms serve split_bf16 trials
-        # too (28 us -> 10 of a 70 us trial at 128^2); dct_precision "fp32" takes them
-        # at every size they serve
-        fast = self.prec == 0 or (self.prec == 3 and max(ep.num_bins_x, ep.num_bins_y) <= 128)
-        self.poisson_ws = PoissonWorkspace(ep.num_bins_x, ep.num_bins_y, self.prec, dev, fast=fast)
+        # (eager or captured) of this design solves on its one stream, by the form
+        # that fast_solve names for trials
+        self.poisson_ws = PoissonWorkspace(ep.num_bins_x, ep.num_bins_y, self.prec, dev,
+                                           fast=fast_solve(self.prec, self.dmap, FAST_TRIAL_SIDE))
         # spatial visiting order of the scattered cells (movable block, then filler
         # block), refreshed every `sort_interval` iterations (refresh_due)
         nm, nf = d.num_movable_nodes, d.num_filler_nodes
