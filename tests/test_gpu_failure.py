@@ -1,10 +1,11 @@
 """Failure detection without a GPU fault.
 
-* The tensor-core GEMM's bounded waits: with the host-set test hook the TMA
-  producer issues no copy, so the MMA warp's wait on the first stage runs out
-  after a short host-set budget; the launch returns, dp_tc_status reports the
-  expired wait, and the context stays usable (the next solve's field maps equal
-  the ones before the failure bit for bit).
+* The bounded waits of the Poisson solve: with the host-set test hook the
+  tensor-core GEMM's TMA producer and the fast transforms' row staging issue no
+  copy, so the MMA warp's wait on the first stage, or the rows', runs out after a
+  short host-set budget; the launch returns, dp_tc_status reports the expired
+  wait, and the context stays usable (the next solve's field maps equal the ones
+  before the failure bit for bit).
 * GP divergence rollback (reference dreamplace/NonLinearPlace.py:534-570,
   641-651): late in GP the movable cells' positions are permuted on the host
   (the occupied spots stay, every net is torn apart), the HPWL jumps while the
@@ -32,30 +33,31 @@ def C():
     return C
 
 
-def _solve(M, precision):
+def _solve(M, precision, fast):
     from dreamplace_b200.electric_potential import poisson_solve
     rng = np.random.RandomState(3)
     rho = torch.from_numpy(rng.uniform(0, 1, size=(M, M)).astype(np.float32)).cuda()
-    ex, ey, energy = poisson_solve(rho, 10.0, 10.0, precision)
+    ex, ey, energy = poisson_solve(rho, 10.0, 10.0, precision, fast=fast)
     torch.cuda.synchronize()
     return ex.clone(), ey.clone(), energy.clone()
 
 
-def test_gemm_bounded_wait_expires_and_context_survives(C):
-    before = _solve(128, "split_bf16")
+@pytest.mark.parametrize("fast", [False, True], ids=["gemm", "fast_transforms"])
+def test_bounded_wait_expires_and_context_survives(C, fast):
+    before = _solve(128, "split_bf16", fast)
     assert C.tc_status() == 0
     try:
         C.tc_set_wait_budget(20_000_000)  # ~10 ms
         C.tc_set_skip_loads(1)
-        _solve(128, "split_bf16")
+        _solve(128, "split_bf16", fast)
         status = C.tc_status()
     finally:
         C.tc_set_skip_loads(0)
         C.tc_set_wait_budget(4_000_000_000)
-    assert status == 2  # the MMA warp's wait for the first operand stage ran out
+    assert status == 2  # the wait for the first operand stage, or for the rows, ran out
     # the context stays usable: the next solve equals the one before (field
-    # maps bit for bit; the energy's per-CTA fp64 partials are added atomically)
-    after = _solve(128, "split_bf16")
+    # maps bit for bit; the energy's per-block fp64 partials are added atomically)
+    after = _solve(128, "split_bf16", fast)
     assert C.tc_status() == 0
     assert torch.equal(before[0], after[0]) and torch.equal(before[1], after[1])
     assert math.isclose(float(before[2]), float(after[2]), rel_tol=1e-12)
