@@ -132,3 +132,29 @@ def test_row_wait_that_expires_with_its_copies_in_flight(C):
         after = poisson_solve(x, 10.0, 10.0, "fp32")
         assert torch.equal(after[0], before[0]) and torch.equal(after[1], before[1])
         assert C.tc_status() == 0
+
+
+@pytest.mark.parametrize("shape", [(64, 128), (1024, 64)])
+def test_interleaved_field_of_the_c_abi(C, shape):
+    """dp_poisson_fft's exy, the field as pairs for hosts that gather both
+    components of a bin, beside its planar maps: the same bits."""
+    import ctypes
+    import os
+    from dreamplace_b200.dct2_fft2 import fft_table
+    from dreamplace_b200.electric_potential import poisson_solve
+    M, N = shape
+    lib = ctypes.CDLL(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "dreamplace_b200",
+                                   "lib", "libdreamplace_b200.so"))
+    x = torch.from_numpy(density(M, N, 2)).cuda()
+    ex, ey, energy = poisson_solve(x, 3.0, 2.0, "fp32")
+    tw = [fft_table(n, x.device) for n in shape]
+    work, exy = torch.empty(3 * M * N, device="cuda"), torch.empty(M, N, 2, device="cuda")
+    e2 = torch.empty(1, dtype=torch.float64, device="cuda")
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    torch.cuda.synchronize()
+    rc = lib.dp_poisson_fft(p(x), M, N, ctypes.c_float(1.0), ctypes.c_float(3.0 / 2.0), p(tw[0]), p(tw[1]), p(work),
+                            None, None, p(exy), p(e2), 1, None)
+    torch.cuda.synchronize()
+    assert rc == 0
+    assert torch.equal(exy[..., 0], ex) and torch.equal(exy[..., 1], ey)
+    assert math.isclose(float(e2), float(energy), rel_tol=1e-12)
