@@ -6,9 +6,9 @@ re-organised for the GPU:
 
 * the objective and its gradient are computed by the hand-written adjoints
   directly (no autograd): WA forward with the pin gather fused in, the density
-  scatter, the four Poisson GEMM launches, the field gather writing the
-  density gradient (scaled by lambda on the device) and the WA backward fused
-  with the pin -> node sum accumulating the wirelength gradient on top;
+  scatter, the Poisson solve (four GEMM launches, or three passes of the fast
+  transforms), the field gather (scaled by lambda on the device) and the assembly
+  of the wirelength gradient's pin -> node sum with it;
 * the Nesterov trial point, move-boundary clamp, preconditioner and the fp64
   step-size estimate run as fused kernels on three rotating slots of (v, u, g)
   buffers, so an accepted step advances a slot index instead of copying;

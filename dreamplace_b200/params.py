@@ -28,7 +28,10 @@ DEFAULTS = {
     "use_bb": 0,
     "num_threads": 8,
     "dtype": "float32",
-    # Poisson-solve arithmetic of this implementation: fp32 | tf32 | bf16 | split_bf16
+    # Poisson-solve arithmetic of this implementation: fp32 | tf32 | bf16 | split_bf16.
+    # On power-of-two grids (64 .. 4096 bins a side) fp32 solves by fast transforms
+    # and is the faster and more exact choice above 128 bins (2.1M cells on 1024^2:
+    # 2,441 GP iterations/s against 2,223); on other grids split_bf16 is the faster
     "dct_precision": "split_bf16",
     # autograd path: 1 keeps only the density map between the electric
     # potential's forward and backward and recomputes the field maps there
