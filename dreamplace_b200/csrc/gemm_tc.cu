@@ -79,6 +79,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int co
   return true;
 }
 
+// waits for what this block has in flight (copies into its shared memory, MMAs
+// that read it) before it may return, also when a wait above gave up: bounded by
+// its own limit, whatever the budget, and without a record
+constexpr long long kTcDrainCycles = 4000000000ll;  // ~2 s at 2 GHz
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return;
+  const long long start = clock64();
+  while (!mbar_try_wait(bar, parity) && clock64() - start <= kTcDrainCycles) {
+  }
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -209,7 +220,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
   if (warp == 0 && lane == 0) {
     // ---- TMA producer ----
     const int skip = g_tc_skip_loads;
-    for (int kb = 0; kb < total_kb && !skip; ++kb) {
+    int kb = 0;
+    for (; kb < total_kb && !skip; ++kb) {
       int s = kb % STAGES, round = kb / STAGES;
       if (round > 0 && !mbar_wait(&empty_bar[s], (round - 1) & 1, 1)) break;
       const int kx = kb * Cfg::kBK;
@@ -223,6 +235,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
         tma_load_2d(sb + Cfg::kBBytes + Cfg::kABytes, &batch.b_lo[z], &full_bar[s], kx, n0);
       }
     }
+    // the ring's last copies (long landed, unless a wait expired)
+    for (int k = kb > STAGES ? kb - STAGES : 0; k < kb; ++k) mbar_drain(&full_bar[k % STAGES], (k / STAGES) & 1);
   } else if (warp == 1 && lane == 0) {
     // ---- MMA issuer ----
     constexpr uint32_t idesc = make_idesc<Cfg::kTF32, BN>();
@@ -301,6 +315,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
       }
     }
   }
+  if (!acc_ok) mbar_drain(acc_bar, 0);
   if (P.energy) {  // ENERGY, or SPECTRAL with the spectral-domain energy
     for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
     if (lane == 0 && e != 0.0) atomicAdd(P.energy, e);

@@ -143,3 +143,25 @@ def test_resume_follows_the_original_trajectory(trials_on_products):
 
 def test_batched_designs_match_single_runs(trials_on_products):
     test_gpu_batch.test_batched_designs_match_single_runs()
+
+
+def test_waits_that_expire_with_copies_in_flight(C):
+    """A wait budget shorter than the copies take: a block that gives up drains
+    its copies and MMAs before it returns, the status says so, and the next solve
+    is what it was."""
+    from dreamplace_b200.electric_potential import poisson_solve
+    for precision, side in (("split_bf16", 136), ("tf32", 1024), ("split_bf16", 1024)):
+        x = torch.from_numpy(placement_map(side, side, 7)).cuda()
+        before = [t.clone() for t in poisson_solve(x, 10.0, 10.0, precision, fast=False)]
+        assert C.tc_status() == 0
+        try:
+            C.tc_set_wait_budget(1)
+            for _ in range(3):
+                poisson_solve(x, 10.0, 10.0, precision, fast=False)
+            status = C.tc_status()
+        finally:
+            C.tc_set_wait_budget(4_000_000_000)
+        assert status in (0, 1, 2, 3)  # the hardware's own wait may outlast the copies
+        after = poisson_solve(x, 10.0, 10.0, precision, fast=False)
+        assert torch.equal(after[0], before[0]) and torch.equal(after[1], before[1])
+        assert C.tc_status() == 0
