@@ -680,7 +680,11 @@ def run_reference(args):
         return 0
     design = make_design(args.design)
     threads = cpu_threads()
-    it = ReferenceCPUIteration(design, threads)
+    try:
+        it = ReferenceCPUIteration(design, threads)
+    except RuntimeError as e:
+        print(json.dumps({"impl": "reference", "unavailable": str(e).replace("\n", " ")}))
+        return 0
     for _ in range(max(args.warmup, 1)):
         it.step()
     steps = args.steps

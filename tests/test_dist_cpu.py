@@ -96,3 +96,17 @@ def test_two_rank_batch_partition_and_gather(num_designs):
     assert slowest > 0
     assert out[world] == pytest.approx(round(num_designs / slowest, 3), rel=1e-3)
     assert out[world + 3] == 1.0
+
+
+def test_reference_arm_without_its_operators_says_so(capsys, monkeypatch):
+    """--impl reference where the reference's CPU operators were not built: one
+    JSON line with the reason, and success."""
+    import json
+    import sys
+    import bench
+    import oracle
+    monkeypatch.setattr(oracle, "load_ref", lambda name: None)
+    monkeypatch.setattr(sys, "argv", ["bench.py", "--impl", "reference", "--design", "cells_10k"])
+    assert bench.main() == 0
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and "not built" in line["unavailable"]
